@@ -112,9 +112,9 @@ static StepArgs split_z(const UppeHandle* h, double z) {
 
 static void free_buffers(UppeHandle* h) {
     void* ptrs[] = {h->q,  h->qi,   h->qf,   h->k1,   h->E,     h->J,      h->scratch, h->opK,  h->opKi, h->kg2,
-                    h->ng, h->tw,   h->w,    h->nlfilt, h->Minv, h->Mfwd, h->kr2_d, h->w2n2_d, h->kg_d, h->red, h->dev_err, h->Minv_tc, h->Mfwd_tc,
+                    h->ng, h->tw,   h->w,    h->nlfilt, h->Bk[0], h->Bk[1], h->Bk[2], h->Bk[3], h->kr2_d, h->w2n2_d, h->kg_d, h->red, h->dev_err, h->Minv_tc, h->Mfwd_tc,
                     h->MfwdT_tc, h->MinvT_tc,
-                    h->adj_q1, h->adj_q2, h->adj_q3, h->adj_lf, h->adj_acc, h->adj_lk, h->adj_mu, h->MfwdT, h->MinvT,
+                    h->adj_q1, h->adj_q2, h->adj_q3, h->adj_lf, h->adj_acc, h->adj_lk, h->adj_mu,
                     h->adj_E[0], h->adj_E[1], h->adj_E[2], h->adj_E[3],
                     h->dred_d, h->rot, h->Atc, h->tw_reg, h->tscr, h->adj_live, h->adj_park};
     for (void* p : ptrs)
@@ -261,10 +261,6 @@ extern "C" int uppe_create(const UppeConfig* cfg, UppeHandle** out) {
     ALLOC(h->tw, ((size_t)1 << h->twLog) * sizeof(float2));
     ALLOC(h->w, (size_t)c.n0 * sizeof(float));
     ALLOC(h->nlfilt, (size_t)c.n0 * sizeof(float));
-    if (c.cylindrical) {
-        ALLOC(h->Minv, (size_t)c.n2 * c.n1 * h->Nk * sizeof(float));
-        ALLOC(h->Mfwd, (size_t)c.n2 * c.n1 * c.n1 * sizeof(float));
-    }
     // the register-resident time pass (M = 256, 512, 1024): its twiddle tables, and its parking
     // scratch for ionizing columns when the medium ionizes
     const bool time_reg = !env && (h->M == 256 || h->M == 512 || h->M == 1024);
@@ -365,8 +361,19 @@ extern "C" int uppe_set_grid(UppeHandle* h, const double* w, const double* kr2, 
                     Minv[((size_t)m * Nr + r) * Nk + k] = (float)(hv * Lambda[k] / Lambda[r]);
                     Mfwd[((size_t)m * Nr + k) * Nr + r] = (float)(hv * Lambda[r] / Lambda[k]);
                 }
-        CUDA_TRY(h, cudaMemcpy(h->Minv, Minv.data(), Minv.size() * sizeof(float), cudaMemcpyHostToDevice));
-        CUDA_TRY(h, cudaMemcpy(h->Mfwd, Mfwd.data(), Mfwd.size() * sizeof(float), cudaMemcpyHostToDevice));
+        // the plain FP32 form's matrices, reduction-major
+        const auto upload_kmajor = [&](int which, const std::vector<float>& M, int NK) -> cudaError_t {
+            std::vector<float> t(hankel_kmajor_len(Nr, Nm));
+            hankel_kmajor(M.data(), Nr, Nm, NK, t.data());
+            cudaError_t e = cudaSuccess;
+            if (!h->Bk[which]) e = cudaMalloc((void**)&h->Bk[which], t.size() * sizeof(float));
+            if (e == cudaSuccess) e = cudaMemcpy(h->Bk[which], t.data(), t.size() * sizeof(float), cudaMemcpyHostToDevice);
+            return e;
+        };
+        if (c.precision == UPPE_PREC_FP32) {
+            CUDA_TRY(h, upload_kmajor(0, Mfwd, Nr));
+            CUDA_TRY(h, upload_kmajor(1, Minv, Nk));
+        }
         // transposed matrices for the adjoint transforms (one azimuthal node)
         if (Nm == 1) {
             std::vector<float> MfT((size_t)Nr * Nr, 0.f), MiT((size_t)Nr * Nr, 0.f);
@@ -375,10 +382,10 @@ extern "C" int uppe_set_grid(UppeHandle* h, const double* w, const double* kr2, 
                     MfT[(size_t)r * Nr + k] = Mfwd[(size_t)k * Nr + r];
                     if (k < Nk) MiT[(size_t)k * Nr + r] = Minv[(size_t)r * Nk + k];
                 }
-            if (!h->MfwdT) CUDA_TRY(h, cudaMalloc((void**)&h->MfwdT, MfT.size() * sizeof(float)));
-            if (!h->MinvT) CUDA_TRY(h, cudaMalloc((void**)&h->MinvT, MiT.size() * sizeof(float)));
-            CUDA_TRY(h, cudaMemcpy(h->MfwdT, MfT.data(), MfT.size() * sizeof(float), cudaMemcpyHostToDevice));
-            CUDA_TRY(h, cudaMemcpy(h->MinvT, MiT.data(), MiT.size() * sizeof(float), cudaMemcpyHostToDevice));
+            if (c.precision == UPPE_PREC_FP32) {
+                CUDA_TRY(h, upload_kmajor(2, MfT, Nr));
+                CUDA_TRY(h, upload_kmajor(3, MiT, Nr));
+            }
             if (c.precision == UPPE_PREC_MIXED) {  // the adjoint transforms on the tensor cores
                 std::vector<uint8_t> t;
                 uppe_split_matrix_tiles(MfT.data(), 1, Nr, Nr, t);

@@ -39,7 +39,13 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 UPPE_DEV float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 UPPE_DEV float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
 UPPE_DEV float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
+// The same product with its roundings spelled out: the same bits whatever code surrounds it
+UPPE_DEV float2 cmul_fixed(float2 a, float2 b) {
+    return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
+}
 UPPE_DEV float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+// a + s b, each component one fused multiply-add whatever surrounds it
+UPPE_DEV float2 caxpy(float2 a, float2 b, float s) { return make_float2(fmaf(b.x, s, a.x), fmaf(b.y, s, a.y)); }
 UPPE_DEV float2 cconj(float2 a) { return make_float2(a.x, -a.y); }
 // multiply by +i / -i
 UPPE_DEV float2 cmul_i(float2 a) { return make_float2(-a.y, a.x); }

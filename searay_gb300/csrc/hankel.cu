@@ -9,18 +9,19 @@
 // The azimuthal FFT (FFT_axis2/IFFT_axis2, fft.cl:401-441) of grids with N2 > 1 runs as a separate
 // DFT pass around the GEMM.
 #include "common.cuh"
+#include "time_common.cuh"
 #include "uppe_internal.h"
 
-#define GBM 32
-#define GBN 64
-#define GBK 16
+#define GBK 16  // reduction elements per shared tile
 
 enum { A_PLAIN = 0, A_QPHASE_IKZ = 1, A_QPHASE = 2, A_SADJ = 3 };
 enum { C_STORE = 0, C_FINISH1 = 1, C_SPEC = 2, C_QADJ = 3, C_FADJ = 4 };
 
 struct GemmArgs {
     const float2* A;  // operand source ([w][r|k][m] layout, row length N1, N2 azimuthal nodes)
-    const float* B;   // [N2][NI][NK]
+    const float* B;   // [N2][KP][LD], reduction-major: B[m][k][i], zero-padded (hankel_kmajor)
+    int KP, LD;
+    int which;        // 0 Mfwd, 1 Minv, 2 Mfwd^T, 3 Minv^T
     OpView op;
     float2* C0;       // store target / q_out / A_out
     float2* C1;       // E (finish) / qf
@@ -31,108 +32,225 @@ struct GemmArgs {
     StepArgs z;
 };
 
-template <int AMODE, int CMODE>
-__global__ void __launch_bounds__(256) k_hankel_gemm(GemmArgs g) {
-    __shared__ float2 As[GBK][GBM + 1];
-    __shared__ __align__(16) float Bs[GBK][GBN + 4];
+// One block: BM frequencies x BN output columns, threads of TM x TN; TX threads along the columns, a
+// thread's columns in groups of four (TX groups apart).  The accumulators of two neighbouring columns
+// share a packed f32x2 register, so a term costs two packed FMAs against the broadcast Re and Im of
+// the field; each sum runs over k in ascending order.  B comes in by 16-byte asynchronous copies and the
+// field (with its propagator factor, formed in registers) by way of the next tile's loads issued
+// before this tile's products, both into the other half of a double buffer: one barrier per 16 k.  The
+// products then go through shared memory, TY rows at a time, to a rolled loop along the columns: the
+// epilogue's code exists once (unrolled over a thread's products it stalled on instruction fetch), its
+// accesses are coalesced, and its operands are loaded four points ahead of the stores.
+//
+// Bound by the FMA pipe: at 2049 x 512 x 512 a product is 1.07e9 FMAs, 28 us at the 39e12/s of 152
+// multiprocessors, about 40 us at the rate an outer product in registers reaches.  Measured there, the propagator
+// factor or the RK stage included: 68 us, against 127 and 120 us with 32 x 64 tiles of 2 x 4 and no copies
+// ahead (512 threads of 2 x 8 against 256 of 4 x 8: 68 against 71 us; scalar FMAs in place of packed
+// ones: the same).
+template <int BM, int BN, int TM, int TN>
+struct GemmShape {
+    static constexpr int TX = BN / TN, TY = BM / TM, T = TX * TY, AE = BM * GBK / T, BE = GBK * BN / 4 / T;
+    static_assert(TY == GBK && TX % 16 == 0 && TN % 4 == 0 && AE >= 1 && BE >= 1, "GEMM shape");
+};
+
+template <int AMODE, int CMODE, int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) k_hankel_gemm(GemmArgs g) {
+    using GS = GemmShape<BM, BN, TM, TN>;
+    __shared__ float2 As[2][GBK][BM + 1];
+    __shared__ __align__(16) float Bs[2][GBK][BN];
+    const int tid = threadIdx.x;
     const int m = blockIdx.z;
-    const int w0 = blockIdx.y * GBM;
-    const int i0 = blockIdx.x * GBN;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    const int w0 = blockIdx.y * BM;
+    const int i0 = blockIdx.x * BN;
+    // a warp covers 16 column groups x 2 rows, so that its B reads are 256 bytes and two rows share them
+    const int lane = tid & 31, warp = tid >> 5;
+    constexpr int WX = GS::TX / 16;
+    const int tx = (lane & 15) + 16 * (warp % WX), ty = (lane >> 4) + 2 * (warp / WX);
     const PhaseArgs pa{g.z.zhi, g.z.zlo, g.z.plain};
-    float2 acc[2][4];
+    f2x accx[TM][TN / 2], accy[TM][TN / 2];
 #pragma unroll
-    for (int r = 0; r < 2; ++r)
+    for (int r = 0; r < TM; ++r)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[r][j] = make_float2(0.f, 0.f);
-    const float* Bm = g.B + (size_t)m * g.NI * g.NK;
-    for (int k0 = 0; k0 < g.NK; k0 += GBK) {
-        for (int e = threadIdx.x; e < GBK * GBM; e += 256) {
-            const int kk = e % GBK, ww = e / GBK;
-            const int w = w0 + ww, k = k0 + kk;
-            float2 v = make_float2(0.f, 0.f);
+        for (int j = 0; j < TN / 2; ++j) accx[r][j] = accy[r][j] = pk2(0.f, 0.f);
+    const float* Bm = g.B + (size_t)m * g.KP * g.LD;
+
+    const auto issue_B = [&](int k0, int half) {
+#pragma unroll
+        for (int s = 0; s < GS::BE; ++s) {
+            const int e = tid + s * GS::T;
+            const int kk = e / (BN / 4), c = 4 * (e % (BN / 4));
+            if (i0 + c < g.LD)
+                cp_async16_time(&Bs[half][kk][c], Bm + (size_t)(k0 + kk) * g.LD + i0 + c);
+            else
+                *reinterpret_cast<float4*>(&Bs[half][kk][c]) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
+    // the field element e = (w, k) of a tile: loads first, the factor when it is stored
+    float2 av[GS::AE], aK[GS::AE];
+    float aki[GS::AE];
+    const auto load_A = [&](int k0) {
+#pragma unroll
+        for (int s = 0; s < GS::AE; ++s) {
+            const int e = tid + s * GS::T;
+            const int w = w0 + e / GBK, k = k0 + e % GBK;
+            av[s] = aK[s] = make_float2(0.f, 0.f);
+            aki[s] = 0.f;
             if (w < g.N0 && k < g.NK) {
                 const size_t idx = ((size_t)w * g.N1 + k) * g.N2 + m;
-                v = g.A[idx];
+                av[s] = g.A[idx];
+                if (AMODE != A_PLAIN) {
+                    aK[s] = g.op.K[idx];
+                    if (g.op.ki) aki[s] = g.op.ki[idx];
+                }
+            }
+        }
+    };
+    const auto store_A = [&](int k0, int half) {
+#pragma unroll
+        for (int s = 0; s < GS::AE; ++s) {
+            const int e = tid + s * GS::T;
+            const int w = w0 + e / GBK, k = k0 + e % GBK;
+            float2 v = av[s];
+            if (AMODE != A_PLAIN && w < g.N0 && k < g.NK) {
+                const float2 kgw = g.op.kg[w];
+                OpPoint o;
+                o.Khi = aK[s].x;
+                o.Klo = aK[s].y;
+                o.kzr = g.op.envelope ? kgw.x : (aK[s].x - kgw.x) + (aK[s].y - kgw.y);
+                o.kzi = aki[s];
                 if (AMODE == A_SADJ) {
                     // conj(D2) v, D2 = (i/2) exp(-i(kz+kg)z) / Re kz
-                    const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
                     const float2 f = cconj(propagator_factor(o, pa, -1.f));
                     v = cscale(cmul_mi(cmul(f, v)), 0.5f / o.kzr);
-                } else if (AMODE != A_PLAIN) {
-                    const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
+                } else {
                     v = cmul(propagator_factor(o, pa, 1.f), v);
                     if (AMODE == A_QPHASE_IKZ) v = op_field(g.op, o, v);
                 }
             }
-            As[kk][ww] = v;
+            As[half][e % GBK][e / GBK] = v;
         }
-        for (int e = threadIdx.x; e < GBK * GBN; e += 256) {
-            const int kk = e % GBK, ii = e / GBK;
-            const int i = i0 + ii, k = k0 + kk;
-            Bs[kk][ii] = (i < g.NI && k < g.NK) ? Bm[(size_t)i * g.NK + k] : 0.f;
+    };
+
+    load_A(0);
+    issue_B(0, 0);
+    store_A(0, 0);
+    int half = 0;
+    for (int k0 = 0; k0 < g.NK; k0 += GBK, half ^= 1) {
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        __syncthreads();  // this tile has landed; the other half has been read
+        const bool more = k0 + GBK < g.NK;
+        if (more) {
+            issue_B(k0 + GBK, half ^ 1);
+            load_A(k0 + GBK);
         }
-        __syncthreads();
 #pragma unroll
         for (int kk = 0; kk < GBK; ++kk) {
-            const float2 a0 = As[kk][ty * 2], a1 = As[kk][ty * 2 + 1];
-            const float4 b = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-            const float bb[4] = {b.x, b.y, b.z, b.w};
+            f2x b[TN / 2];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                acc[0][j].x = fmaf(a0.x, bb[j], acc[0][j].x);
-                acc[0][j].y = fmaf(a0.y, bb[j], acc[0][j].y);
-                acc[1][j].x = fmaf(a1.x, bb[j], acc[1][j].x);
-                acc[1][j].y = fmaf(a1.y, bb[j], acc[1][j].y);
+            for (int q = 0; q < TN / 4; ++q) {
+                const float4 v = *reinterpret_cast<const float4*>(&Bs[half][kk][4 * (q * GS::TX + tx)]);
+                b[2 * q] = pk2(v.x, v.y);
+                b[2 * q + 1] = pk2(v.z, v.w);
+            }
+#pragma unroll
+            for (int r = 0; r < TM; ++r) {
+                const float2 a = As[half][kk][ty * TM + r];
+                const f2x ax = pk2(a.x, a.x), ay = pk2(a.y, a.y);
+#pragma unroll
+                for (int j = 0; j < TN / 2; ++j) {
+                    accx[r][j] = fma2(ax, b[j], accx[r][j]);
+                    accy[r][j] = fma2(ay, b[j], accy[r][j]);
+                }
             }
         }
-        __syncthreads();
+        if (more) store_A(k0 + GBK, half ^ 1);
     }
+    // ---- epilogue ----
+    float2* stage = reinterpret_cast<float2*>(&Bs[0][0][0]);  // TY rows of BN products
+    const bool need_a = CMODE == C_SPEC && (g.spec_mode == SPEC_STAGE1 || g.spec_mode == SPEC_STAGE23);
+    const bool need_b = CMODE == C_SPEC && (g.spec_mode == SPEC_STAGE23 || g.spec_mode == SPEC_FINISH);
+#pragma unroll 1
+    for (int r = 0; r < TM; ++r) {
+        __syncthreads();  // the last tile's products, or the previous rows, have been read
 #pragma unroll
-    for (int r = 0; r < 2; ++r) {
-        const int w = w0 + ty * 2 + r;
-        if (w >= g.N0) continue;
-        const float cond = (w < g.op.ncond) ? 0.f : 1.f;
+        for (int j = 0; j < TN / 2; ++j) {
+            f2x vx = accx[0][j], vy = accy[0][j];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int i = i0 + tx * 4 + j;
-            if (i >= g.NI) continue;
-            const size_t idx = ((size_t)w * g.N1 + i) * g.N2 + m;
-            const float2 v = acc[r][j];
-            if (CMODE == C_STORE) {
-                g.C0[idx] = v;
-            } else if (CMODE == C_QADJ || CMODE == C_FADJ) {
-                const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
-                float2 r = cmul(cconj(propagator_factor(o, pa, 1.f)), v);
-                if (CMODE == C_QADJ) r = cmul(cconj(op_ikz(o)), r);
-                g.C0[idx] = r;
-            } else if (CMODE == C_FINISH1) {
-                const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
-                if (g.C0) g.C0[idx] = v;
-                g.C1[idx] = op_field(g.op, o, v);
-            } else {
-                const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
-                float2 f = propagator_factor(o, pa, -1.f);
-                float2 s = cscale(cmul_i(cmul(f, v)), 0.5f / o.kzr);
-                switch (g.spec_mode) {
-                    case SPEC_STORE_K:
-                        g.C0[idx] = s;
-                        break;
-                    case SPEC_STAGE1: {
-                        float2 a = g.qi[idx];
-                        g.C1[idx] = cadd(a, cscale(s, g.Cs));
-                        g.C0[idx] = cscale(cadd(a, cscale(s, g.Ce)), cond);
-                    } break;
-                    case SPEC_STAGE23: {
-                        float2 a = g.qi[idx];
-                        float2 b = g.C1[idx];
-                        g.C1[idx] = cadd(b, cscale(s, g.Cs));
-                        g.C0[idx] = cscale(cadd(a, cscale(s, g.Ce)), cond);
-                    } break;
-                    default: {
-                        float2 b = g.C1[idx];
-                        g.C0[idx] = cscale(cadd(b, cscale(s, g.Cs)), cond);
-                    } break;
+            for (int rr = 1; rr < TM; ++rr)
+                if (r == rr) {
+                    vx = accx[rr][j];
+                    vy = accy[rr][j];
+                }
+            const float2 x = up2(vx), y = up2(vy);
+            const int c = 4 * ((j / 2) * GS::TX + tx) + 2 * (j % 2);
+            *reinterpret_cast<float4*>(&stage[ty * BN + c]) = make_float4(x.x, y.x, x.y, y.y);
+        }
+        __syncthreads();
+        constexpr int NE = GS::TY * BN / GS::T, U = NE < 4 ? NE : 4;
+#pragma unroll 1
+        for (int e0 = 0; e0 < NE; e0 += U) {
+            float2 v[U], K[U], qa[U], qb[U];
+            float ki[U];
+            size_t idx[U];
+            bool in[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int e = tid + (e0 + u) * GS::T;
+                const int c = e % BN, w = w0 + (e / BN) * TM + r, i = i0 + c;
+                in[u] = w < g.N0 && i < g.NI;
+                idx[u] = ((size_t)w * g.N1 + i) * g.N2 + m;
+                v[u] = stage[(e / BN) * BN + c];
+                K[u] = qa[u] = qb[u] = make_float2(0.f, 0.f);
+                ki[u] = 0.f;
+                if (CMODE != C_STORE && in[u]) {
+                    K[u] = g.op.K[idx[u]];
+                    if (g.op.ki) ki[u] = g.op.ki[idx[u]];
+                    if (need_a) qa[u] = g.qi[idx[u]];
+                    if (need_b) qb[u] = g.C1[idx[u]];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (!in[u]) continue;
+                const int w = w0 + ((tid + (e0 + u) * GS::T) / BN) * TM + r;
+                if constexpr (CMODE == C_STORE) {
+                    g.C0[idx[u]] = v[u];
+                    continue;
+                }
+                const float cond = (w < g.op.ncond) ? 0.f : 1.f;
+                const float2 kgw = g.op.kg[w];
+                OpPoint o;
+                o.Khi = K[u].x;
+                o.Klo = K[u].y;
+                o.kzr = g.op.envelope ? kgw.x : (K[u].x - kgw.x) + (K[u].y - kgw.y);
+                o.kzi = ki[u];
+                if constexpr (CMODE == C_QADJ || CMODE == C_FADJ) {
+                    float2 c = cmul(cconj(propagator_factor(o, pa, 1.f)), v[u]);
+                    if (CMODE == C_QADJ) c = cmul(cconj(op_ikz(o)), c);
+                    g.C0[idx[u]] = c;
+                } else if constexpr (CMODE == C_FINISH1) {
+                    if (g.C0) g.C0[idx[u]] = v[u];
+                    g.C1[idx[u]] = op_field(g.op, o, v[u]);
+                } else if constexpr (CMODE == C_SPEC) {
+                    const float2 f = propagator_factor(o, pa, -1.f);
+                    const float2 s = cscale(cmul_i(cmul_fixed(f, v[u])), 0.5f / o.kzr);
+                    switch (g.spec_mode) {
+                        case SPEC_STORE_K:
+                            g.C0[idx[u]] = s;
+                            break;
+                        case SPEC_STAGE1:
+                            g.C1[idx[u]] = caxpy(qa[u], s, g.Cs);
+                            g.C0[idx[u]] = cscale(caxpy(qa[u], s, g.Ce), cond);
+                            break;
+                        case SPEC_STAGE23:
+                            g.C1[idx[u]] = caxpy(qb[u], s, g.Cs);
+                            g.C0[idx[u]] = cscale(caxpy(qa[u], s, g.Ce), cond);
+                            break;
+                        default:
+                            g.C0[idx[u]] = cscale(caxpy(qb[u], s, g.Cs), cond);
+                            break;
+                    }
                 }
             }
         }
@@ -174,16 +292,54 @@ cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* 
                              float2* C1, const float2* qi, int NI, int NK, int spec_mode, float Cs, float Ce,
                              StepArgs z);
 
-// Mixed-precision form: tensor-core GEMM (hankel_tc.cu); plain FP32 form: the FP32 SIMT GEMM below.
+size_t hankel_kmajor_len(int N1, int N2) {
+    const size_t KP = (size_t)(N1 + GBK - 1) / GBK * GBK, LD = (size_t)(N1 + 3) / 4 * 4;
+    return (size_t)N2 * KP * LD;
+}
+
+// The matrix M[m][i][k] (rows of NK) as the FP32 GEMM reads it, out[m][k][i], zero-padded to KP x LD.
+void hankel_kmajor(const float* M, int N1, int N2, int NK, float* out) {
+    const size_t KP = (size_t)(N1 + GBK - 1) / GBK * GBK, LD = (size_t)(N1 + 3) / 4 * 4;
+    for (size_t e = 0; e < (size_t)N2 * KP * LD; ++e) out[e] = 0.f;
+    for (int m = 0; m < N2; ++m)
+        for (int i = 0; i < N1; ++i)
+            for (int k = 0; k < NK; ++k) out[((size_t)m * KP + k) * LD + i] = M[((size_t)m * N1 + i) * NK + k];
+}
+
+template <int AMODE, int CMODE, int BM, int BN, int TM, int TN>
+static cudaError_t run_simt_shape(UppeHandle* h, const GemmArgs& g) {
+    dim3 grid((g.NI + BN - 1) / BN, (g.N0 + BM - 1) / BM, g.N2);
+    k_hankel_gemm<AMODE, CMODE, BM, BN, TM, TN><<<grid, (BM / TM) * (BN / TN), 0, h->stream>>>(g);
+    return cudaGetLastError();
+}
+
+// The plain FP32 GEMM.  Wide tiles reuse each field element (and its propagator factor) for more columns
+// and need fewer shared loads per FMA, narrow ones make more blocks: the widest whose blocks still cover
+// three quarters of the multiprocessors, and 16 x 64 below that.  Step times in us with tiles of 256 | 128 |
+// 64 | 16 x 64 (the chosen one starred): 2049 x 512 609* | 693 | 705 | 821, 1025 x 512 574 | 381* | 406 |
+// 493, 513 x 512 551 | 364 | 272* | 288, 257 x 256 316 | 214 | 168 | 132*, 257 x 64 145 | 108 | 92 | 78*.
+template <int AMODE, int CMODE>
+static cudaError_t run_simt(UppeHandle* h, GemmArgs& g) {
+    if (!h->Bk[g.which]) return cudaErrorInvalidValue;
+    g.B = h->Bk[g.which];
+    g.KP = (h->N1 + GBK - 1) / GBK * GBK;
+    g.LD = (h->N1 + 3) / 4 * 4;
+    h->launches++;
+    const auto blocks = [&](int bn) { return (long)((g.NI + bn - 1) / bn) * ((g.N0 + 31) / 32) * g.N2; };
+    const long want = (long)h->num_sms * 3 / 4;
+    if (g.NI > 128 && blocks(256) >= want) return run_simt_shape<AMODE, CMODE, 32, 256, 2, 8>(h, g);
+    if (g.NI > 64 && blocks(128) >= want) return run_simt_shape<AMODE, CMODE, 32, 128, 2, 4>(h, g);
+    if (blocks(64) >= want) return run_simt_shape<AMODE, CMODE, 32, 64, 2, 4>(h, g);
+    return run_simt_shape<AMODE, CMODE, 16, 64, 1, 4>(h, g);
+}
+
+// Mixed-precision form: tensor-core GEMM (hankel_tc.cu); plain FP32 form: the FP32 SIMT GEMM above.
 template <int AMODE, int CMODE>
 static cudaError_t run_gemm(UppeHandle* h, GemmArgs& g) {
     if (h->cfg.precision == UPPE_PREC_MIXED)
-        return launch_hankel_tc(h, AMODE, CMODE, g.A, g.B == h->Minv ? 1 : 0, g.C0, g.C1, g.qi, g.NI, g.NK,
-                                g.spec_mode, g.Cs, g.Ce, g.z);
-    dim3 grid((g.NI + GBN - 1) / GBN, (g.N0 + GBM - 1) / GBM, g.N2);
-    h->launches++;
-    k_hankel_gemm<AMODE, CMODE><<<grid, 256, 0, h->stream>>>(g);
-    return cudaGetLastError();
+        return launch_hankel_tc(h, AMODE, CMODE, g.A, g.which, g.C0, g.C1, g.qi, g.NI, g.NK, g.spec_mode, g.Cs, g.Ce,
+                                g.z);
+    return run_simt<AMODE, CMODE>(h, g);
 }
 
 static GemmArgs base_args(UppeHandle* h, StepArgs z) {
@@ -200,7 +356,7 @@ static GemmArgs base_args(UppeHandle* h, StepArgs z) {
 cudaError_t launch_real_cyl(UppeHandle* h, int mode, const float2* src, float2* A_out, StepArgs z) {
     GemmArgs g = base_args(h, z);
     g.A = src;
-    g.B = h->Minv;
+    g.which = 1;
     g.NI = h->N1;
     g.NK = h->Nk;
     cudaError_t err;
@@ -237,7 +393,7 @@ cudaError_t launch_real_cyl(UppeHandle* h, int mode, const float2* src, float2* 
 cudaError_t launch_spec_cyl(UppeHandle* h, int mode, const float2* src_real, float2* q_out, float2* qf_io,
                             const float2* qi, float Cs, float Ce, StepArgs z, const StepArgs* z_next) {
     GemmArgs g = base_args(h, z);
-    g.B = h->Mfwd;
+    g.which = 0;
     g.NI = h->N1;
     g.NK = h->N1;
     g.A = src_real;
@@ -267,17 +423,6 @@ cudaError_t launch_spec_cyl(UppeHandle* h, int mode, const float2* src_real, flo
 // Adjoint transverse transforms on cylindrical grids (one azimuthal node) with the transposed folded
 // matrices: ADJ_S / ADJ_LOAD apply Mfwd^T, ADJ_E / ADJ_FIN apply Minv^T; the tensor-core GEMM in the
 // mixed-precision form, the FP32 SIMT GEMM in the plain form.
-template <int AMODE, int CMODE>
-static cudaError_t run_gemm_adj(UppeHandle* h, GemmArgs& g) {
-    if (h->cfg.precision == UPPE_PREC_MIXED)
-        return launch_hankel_tc(h, AMODE, CMODE, g.A, g.B == h->MfwdT ? 2 : 3, g.C0, g.C1, g.qi, g.NI, g.NK,
-                                g.spec_mode, g.Cs, g.Ce, g.z);
-    dim3 grid((g.NI + GBN - 1) / GBN, (g.N0 + GBM - 1) / GBM, g.N2);
-    h->launches++;
-    k_hankel_gemm<AMODE, CMODE><<<grid, 256, 0, h->stream>>>(g);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_adj_cyl(UppeHandle* h, int mode, const float2* in, float2* out, StepArgs z) {
     GemmArgs g = base_args(h, z);
     g.A = in;
@@ -286,16 +431,16 @@ cudaError_t launch_adj_cyl(UppeHandle* h, int mode, const float2* in, float2* ou
     g.NK = h->N1;
     switch (mode) {
         case ADJ_S:
-            g.B = h->MfwdT;
-            return run_gemm_adj<A_SADJ, C_STORE>(h, g);
+            g.which = 2;
+            return run_gemm<A_SADJ, C_STORE>(h, g);
         case ADJ_LOAD:
-            g.B = h->MfwdT;
-            return run_gemm_adj<A_PLAIN, C_STORE>(h, g);
+            g.which = 2;
+            return run_gemm<A_PLAIN, C_STORE>(h, g);
         case ADJ_E:
-            g.B = h->MinvT;
-            return run_gemm_adj<A_PLAIN, C_QADJ>(h, g);
+            g.which = 3;
+            return run_gemm<A_PLAIN, C_QADJ>(h, g);
         default:
-            g.B = h->MinvT;
-            return run_gemm_adj<A_PLAIN, C_FADJ>(h, g);
+            g.which = 3;
+            return run_gemm<A_PLAIN, C_FADJ>(h, g);
     }
 }

@@ -75,9 +75,9 @@ struct UppeHandle {
     float2* adj_park; // its parking scratch for e(t) ([S][M]) when tscr is NULL, or NULL
     float* w;        // omega per bin (FP32)
     float* nlfilt;   // NL filter per bin
-    float* Minv;     // cylindrical: [N2][Nr][Nk]
-    float* Mfwd;     // cylindrical: [N2][Nr][Nr] (rows >= Nk zero)
-    uint8_t* Minv_tc; // the same, split into bf16 hi/lo tensor-core tiles (mixed form)
+    // cylindrical transform matrices, Minv[r][k] (k < Nk) and Mfwd[k][r] (rows >= Nk zero) per azimuthal mode:
+    float* Bk[4];     // plain FP32 form: Mfwd, Minv, Mfwd^T, Minv^T, reduction-major (hankel_kmajor), or NULL
+    uint8_t* Minv_tc; // mixed form: split into bf16 hi/lo tensor-core tiles
     uint8_t* Mfwd_tc;
     uint8_t* MfwdT_tc; // the transposed matrices of the adjoint transforms, split the same way
     uint8_t* MinvT_tc;
@@ -109,8 +109,6 @@ struct UppeHandle {
     int kept_valid;        // adj_E[0..3] hold the stage fields of the step taken by uppe_rk4_step_keep
     double kept_z, kept_dz;
     long long kept_mat;
-    float* MfwdT;          // cylindrical adjoint: [Nr][Nr], MfwdT[r][k] = Mfwd[k][r]
-    float* MinvT;          // [Nr][Nr], MinvT[k][r] = Minv[r][k] for k < Nk, 0 beyond
     double* dred_d;        // device accumulator of d(loss)/d(chi3/nref)
     long long mat_version; // incremented by every uppe_set_material
     int E_valid;           // E holds T^-1(i kz e^{..} qi) for (E_z, E_mat): reusable by the next step
@@ -212,6 +210,8 @@ cudaError_t uppe_configure_time_adj_kernel(size_t smem_bytes);
 cudaError_t launch_adj_cyl(UppeHandle* h, int mode, const float2* in, float2* out, StepArgs z);
 
 // ---- cylindrical transverse transform (hankel.cu) ----
+size_t hankel_kmajor_len(int N1, int N2);
+void hankel_kmajor(const float* M, int N1, int N2, int NK, float* out);
 cudaError_t launch_real_cyl(UppeHandle* h, int mode, const float2* src, float2* A_out, StepArgs z);
 cudaError_t launch_spec_cyl(UppeHandle* h, int mode, const float2* src_real, float2* q_out, float2* qf_io,
                             const float2* qi, float Cs, float Ce, StepArgs z, const StepArgs* z_next = nullptr);
