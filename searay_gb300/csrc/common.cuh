@@ -43,6 +43,10 @@ UPPE_DEV float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * 
 UPPE_DEV float2 cmul_fixed(float2 a, float2 b) {
     return make_float2(fmaf(a.x, b.x, -__fmul_rn(a.y, b.y)), fmaf(a.x, b.y, __fmul_rn(a.y, b.x)));
 }
+// conj(f) a for a unit phasor f = (cos, sin), roundings spelled out
+UPPE_DEV float2 cmul_conj_fixed(float2 f, float2 a) {
+    return make_float2(fmaf(f.x, a.x, __fmul_rn(f.y, a.y)), fmaf(-f.y, a.x, __fmul_rn(f.x, a.y)));
+}
 UPPE_DEV float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
 // a + s b, each component one fused multiply-add whatever surrounds it
 UPPE_DEV float2 caxpy(float2 a, float2 b, float s) { return make_float2(fmaf(b.x, s, a.x), fmaf(b.y, s, a.y)); }
@@ -168,6 +172,25 @@ UPPE_DEV float2 propagator_factor(const OpPoint& o, PhaseArgs pa, float sign) {
     const float amp = expf(-sign * o.kzi * (pa.zhi + pa.zlo));
     return make_float2(amp * c, sign * amp * s);
 }
+
+// The two propagator factors of a stage update in the usual case, known when the kernel is chosen: the mixed
+// form in a real medium (float-float phase, Im kz = 0).  The branches of propagator_factor and its
+// full-range sincos and exp then leave the kernel, and where both factors are at the same z (`same`, half
+// of the stage updates) one phasor serves both.  The same bits as the general form gives there.
+struct PropagatorPair {
+    float c, s;  // exp(i(kz + kg) z) at the last z asked
+    // exp(-i(kz + kg) z) a
+    UPPE_DEV float2 backward(const OpPoint& o, const PhaseArgs& z, float2 a) {
+        __sincosf(ff_phase(o.Khi, o.Klo, z.zhi, z.zlo), &s, &c);
+        return cmul_conj_fixed(make_float2(c, s), a);
+    }
+    // i kz exp(i(kz + kg) z) q; the products by kz stay products when they meet a sum
+    UPPE_DEV float2 field(const OpPoint& o, const PhaseArgs& z, bool same, float2 q) {
+        if (!same) __sincosf(ff_phase(o.Khi, o.Klo, z.zhi, z.zlo), &s, &c);
+        const float2 e = cmul_fixed(make_float2(c, s), q);
+        return make_float2(-__fmul_rn(o.kzr, e.y), __fmul_rn(o.kzr, e.x));
+    }
+};
 
 // Ask the memory system to bring `bytes` (a multiple of 16, 16-byte aligned) into L2 ahead of use.
 UPPE_DEV void prefetch_l2(const void* p, size_t bytes) {

@@ -450,8 +450,14 @@ UPPE_DEV void stage_async16(float2* smem_dst, const float2* gsrc) {
 // next slice's current is copied into the staging buffer during this slice's inverse transform;
 // the pointwise operands stream through the ring during the forward transform and the pointwise
 // loop.
+//
+// Bound by instruction issue (68 % of the issue slots, 262 thread instructions per point at 128 x 128,
+// about 100 of them pointwise).  FAST (PropagatorPair: the mixed form in a real medium) takes the branches,
+// the full-range sincos and exp and half of the phasors of two of the four stages out of the loop, and
+// with that shorter body four registers a trip pay off: 513 x 128 x 128, the pass with its zero-current
+// slices 117.8 -> 107.1 us per evaluation (FAST alone 110.5, with ROT = 4 108.9).  The general form keeps ROT = 2.
 // ---------------------------------------------------------------------------------------------
-template <int LN1, int LN2>
+template <int LN1, int LN2, bool FAST>
 __global__ void __launch_bounds__(RegSlice<LN1, LN2>::T, 1)
     k_fused_reg(int mode, const float2* __restrict__ J, OpView opv, float2* __restrict__ qi_out,
                 float2* __restrict__ qf, const float2* __restrict__ qi, float2* __restrict__ E, float Cs, float Ce,
@@ -466,6 +472,7 @@ __global__ void __launch_bounds__(RegSlice<LN1, LN2>::T, 1)
     const PhaseArgs pr{z_rhs.zhi, z_rhs.zlo, z_rhs.plain};
     const PhaseArgs pn{z_next.zhi, z_next.zlo, z_next.plain};
     const bool need_qi = (mode != SPEC_FINISH), need_qf = (mode != SPEC_STAGE1);
+    const bool same_z = pr.zhi == pn.zhi && pr.zlo == pn.zlo;
 
     // the current of slice iw -> staging buffer, 16-byte chunks, consecutive threads on consecutive chunks
     auto issue_J = [&](int iw) {
@@ -521,13 +528,14 @@ __global__ void __launch_bounds__(RegSlice<LN1, LN2>::T, 1)
 
         const float cond = (iw < 4) ? 0.f : 1.f;
         const float2 kgw = opv.kg[iw];
-        // Two registers per trip, then the register array rotates by two, so the loop body exists
-        // once in the code rather than sixteen times (the fully unrolled form thrashed the
-        // instruction cache); after eight trips w is back in order.
+        // ROT registers per trip, then the register array rotates by ROT, so the loop body exists
+        // ROT times in the code rather than sixteen (the fully unrolled form thrashed the
+        // instruction cache); after 16 / ROT trips w is back in order.
+        constexpr int ROT = FAST ? 4 : 2;
 #pragma unroll 1
-        for (int r0 = 0; r0 < 16; r0 += 2) {
+        for (int r0 = 0; r0 < 16; r0 += ROT) {
 #pragma unroll
-            for (int d = 0; d < 2; ++d) {
+            for (int d = 0; d < ROT; ++d) {
                 const int r = r0 + d;
                 asm volatile("cp.async.wait_group %0;\n" ::"n"(FP::NSLOT - 1) : "memory");
                 __syncwarp(FP::WMASK);  // the copying lane's data is visible to its neighbour
@@ -540,32 +548,41 @@ __global__ void __launch_bounds__(RegSlice<LN1, LN2>::T, 1)
                 o.Khi = K.x;
                 o.Klo = K.y;
                 o.kzr = (K.x - kgw.x) + (K.y - kgw.y);
-                o.kzi = opv.ki ? opv.ki[idx] : 0.f;
+                o.kzi = !FAST && opv.ki ? opv.ki[idx] : 0.f;
                 // S and the RK stage (the arithmetic of spec_update, on staged values)
-                const float2 f = propagator_factor(o, pr, -1.f);
-                const float2 sv = cscale(cmul_i(cmul(f, w[d])), 0.5f / o.kzr);
+                PropagatorPair pp;
+                float2 sv;
+                if constexpr (FAST)
+                    sv = cscale(cmul_i(pp.backward(o, pr, w[d])), 0.5f / o.kzr);
+                else
+                    sv = cscale(cmul_i(cmul(propagator_factor(o, pr, -1.f), w[d])), 0.5f / o.kzr);
                 float2 qw;
                 if (mode == SPEC_STAGE1) {
-                    qf[idx] = cadd(qiv, cscale(sv, Cs));
-                    qw = cscale(cadd(qiv, cscale(sv, Ce)), cond);
+                    qf[idx] = caxpy(qiv, sv, Cs);
+                    qw = cscale(caxpy(qiv, sv, Ce), cond);
                     if (q_store) q_store[idx] = qw;
                 } else if (mode == SPEC_STAGE23) {
-                    qf[idx] = cadd(qfv, cscale(sv, Cs));
-                    qw = cscale(cadd(qiv, cscale(sv, Ce)), cond);
+                    qf[idx] = caxpy(qfv, sv, Cs);
+                    qw = cscale(caxpy(qiv, sv, Ce), cond);
                     if (q_store) q_store[idx] = qw;
                 } else {
-                    qw = cscale(cadd(qfv, cscale(sv, Cs)), cond);
+                    qw = cscale(caxpy(qfv, sv, Cs), cond);
                     qi_out[idx] = qw;
                 }
-                w[d] = cmul(op_ikz(o), cmul(propagator_factor(o, pn, 1.f), qw));
+                if constexpr (FAST)
+                    w[d] = pp.field(o, pn, same_z, qw);
+                else
+                    w[d] = cmul(op_ikz(o), cmul(propagator_factor(o, pn, 1.f), qw));
                 __syncwarp(FP::WMASK);  // both lanes of the pair have read the slot before it is refilled
                 issue(r + FP::NSLOT);
             }
-            const float2 t0 = w[0], t1 = w[1];
+            float2 t[ROT];
 #pragma unroll
-            for (int i = 0; i < 14; ++i) w[i] = w[i + 2];
-            w[14] = t0;
-            w[15] = t1;
+            for (int i = 0; i < ROT; ++i) t[i] = w[i];
+#pragma unroll
+            for (int i = 0; i < 16 - ROT; ++i) w[i] = w[i + ROT];
+#pragma unroll
+            for (int i = 0; i < ROT; ++i) w[16 - ROT + i] = t[i];
         }
         __syncthreads();  // every ring slot has been read: the staging buffer takes the next current
         if (iw + (int)gridDim.x < n0) issue_J(iw + gridDim.x);

@@ -4,13 +4,19 @@
 template <int LN1, int LN2>
 struct FusedReg {
     static cudaError_t configure() {
-        return cudaFuncSetAttribute(k_fused_reg<LN1, LN2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    FusedPlan<LN1, LN2>::SMEM);
+        cudaError_t e = cudaFuncSetAttribute(k_fused_reg<LN1, LN2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             FusedPlan<LN1, LN2>::SMEM);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k_fused_reg<LN1, LN2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     FusedPlan<LN1, LN2>::SMEM);
+        return e;
     }
     static cudaError_t run(UppeHandle* h, int mode, float Cs, float Ce, StepArgs z_rhs, StepArgs z_next, int n) {
         using RS = RegSlice<LN1, LN2>;
         const int grid = n < h->num_sms ? n : h->num_sms;  // persistent: one CTA per multiprocessor
-        k_fused_reg<LN1, LN2><<<grid, RS::T, FusedPlan<LN1, LN2>::SMEM, h->stream>>>(
+        const auto kernel = (h->cfg.precision == UPPE_PREC_MIXED && !h->complex_medium) ? k_fused_reg<LN1, LN2, true>
+                                                                                         : k_fused_reg<LN1, LN2, false>;
+        kernel<<<grid, RS::T, FusedPlan<LN1, LN2>::SMEM, h->stream>>>(
             mode, h->J, uppe_op_view(h), h->qi, h->qf, h->qi, h->E, Cs, Ce, h->tw, h->twLog, z_rhs, z_next, n,
             h->stage_q);
         return cudaGetLastError();
