@@ -48,10 +48,7 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
     const size_t col0 = (size_t)blockIdx.x * NC;
 
     // ---- stage the NC half spectra of E into the column buffers ----
-    for (int i = tid; i < (M + 1) * NC; i += G::THREADS) {
-        const int c = i & (NC - 1), k = i / NC;
-        cp_async8(&sm[c * LD + k], &E[(size_t)k * S + col0 + c]);
-    }
+    tr_each_point<LOGM>(tid, S, col0, [&](int, int, size_t o, int p) { cp_async8(&sm[p], &E[o]); });
     asm volatile("cp.async.commit_group;\n" ::);
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
@@ -103,10 +100,8 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
     __syncthreads();  // every column's exchange reads of its buffer are done
 
     // ---- stage G of the columns this pass takes ----
-    for (int i = tid; i < (M + 1) * NC; i += G::THREADS) {
-        const int c = i & (NC - 1), k = i / NC;
-        if (!grp_live[c / CA]) cp_async8(&sm[c * LD + k], &Gc[(size_t)k * S + col0 + c]);
-    }
+    const bool take = !grp_live[(tid & (NC - 1)) / CA];  // the group of this thread's column
+    if (take) tr_each_point<LOGM>(tid, S, col0, [&](int, int, size_t o, int p) { cp_async8(&sm[p], &Gc[o]); });
     asm volatile("cp.async.commit_group;\n" ::);
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
@@ -149,14 +144,13 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
         for (int i = 0; i < G::THREADS / 32; ++i) b += red_sh[i];
         if (b != 0.0) atomicAdd(dred, b);
     }
-    for (int i = tid; i < (M + 1) * NC; i += G::THREADS) {
-        const int c = i & (NC - 1), k = i / NC;
-        if (grp_live[c / CA]) continue;
-        if (tp.atc)  // the operand tiles of the Minv^T transform that follows
-            tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + c), sm[c * LD + k]);
-        else
-            gE[(size_t)k * S + col0 + c] = sm[c * LD + k];
-    }
+    if (!take) return;
+    if (tp.atc)  // the operand tiles of the Minv^T transform that follows
+        tr_each_point<LOGM>(tid, S, col0, [&](int k, int c, size_t, int p) {
+            tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + c), sm[p]);
+        });
+    else
+        tr_each_point<LOGM>(tid, S, col0, [&](int, int, size_t o, int p) { gE[o] = sm[p]; });
 }
 
 // ---- host side ----

@@ -49,10 +49,7 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
 
     pdl_begin();
     // ---- stage the NC half spectra X[k][c] (k <= M) into the column buffers ----
-    for (int i = tid; i < (M + 1) * NC; i += G::THREADS) {
-        const int c = i & (NC - 1), k = i / NC;
-        cp_async8(&sm[c * LD + k], &E[(size_t)k * S + col0 + c]);
-    }
+    tr_each_point<LOGM>(tid, S, col0, [&](int, int, size_t o, int p) { cp_async8(&sm[p], &E[o]); });
     asm volatile("cp.async.commit_group;\n" ::);
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncthreads();
@@ -202,13 +199,12 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
 
     // ---- write J back: rows of NC columns ----
     __syncthreads();
-    for (int i = tid; i < (M + 1) * NC; i += G::THREADS) {
-        const int c = i & (NC - 1), k = i / NC;
-        if (tp.atc)
-            tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + c), sm[c * LD + k]);
-        else
-            Jout[(size_t)k * S + col0 + c] = sm[c * LD + k];
-    }
+    if (tp.atc)
+        tr_each_point<LOGM>(tid, S, col0, [&](int k, int c, size_t, int p) {
+            tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + c), sm[p]);
+        });
+    else
+        tr_each_point<LOGM>(tid, S, col0, [&](int, int, size_t o, int p) { Jout[o] = sm[p]; });
 }
 
 // ---- host side ----
