@@ -116,7 +116,7 @@ static void free_buffers(UppeHandle* h) {
                     h->MfwdT_tc, h->MinvT_tc,
                     h->adj_q1, h->adj_q2, h->adj_q3, h->adj_lf, h->adj_acc, h->adj_lk, h->adj_mu,
                     h->adj_E[0], h->adj_E[1], h->adj_E[2], h->adj_E[3],
-                    h->dred_d, h->rot, h->Atc, h->tw_reg, h->tscr, h->adj_live, h->adj_park};
+                    h->dred_d, h->rot, h->Atc, h->tw_line, h->tw_reg, h->tscr, h->adj_live, h->adj_park};
     for (void* p : ptrs)
         if (p) cudaFree(p);
 }
@@ -261,6 +261,7 @@ extern "C" int uppe_create(const UppeConfig* cfg, UppeHandle** out) {
     ALLOC(h->tw, ((size_t)1 << h->twLog) * sizeof(float2));
     ALLOC(h->w, (size_t)c.n0 * sizeof(float));
     ALLOC(h->nlfilt, (size_t)c.n0 * sizeof(float));
+    if (h->slice_big) ALLOC(h->tw_line, big_line_table_len() * sizeof(float4));
     // the register-resident time pass (M = 256, 512, 1024): its twiddle tables, and its parking
     // scratch for ionizing columns when the medium ionizes
     const bool time_reg = !env && (h->M == 256 || h->M == 512 || h->M == 1024);
@@ -290,6 +291,11 @@ extern "C" int uppe_create(const UppeConfig* cfg, UppeHandle** out) {
         std::vector<float2> twr(time_reg_table_len(h->M));
         time_reg_tables(h->M, twr.data());
         e = cudaMemcpy(h->tw_reg, twr.data(), twr.size() * sizeof(float2), cudaMemcpyHostToDevice);
+    }
+    if (e == cudaSuccess && h->tw_line) {
+        std::vector<float4> twl(big_line_table_len());
+        big_line_tables(twl.data());
+        e = cudaMemcpy(h->tw_line, twl.data(), twl.size() * sizeof(float4), cudaMemcpyHostToDevice);
     }
     if (e == cudaSuccess) e = cudaMemset(h->dev_err, 0, sizeof(int));
     // Allow the kernels that stage a whole slice / time tile in shared memory the full 227 KB; each

@@ -38,6 +38,21 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
 
 UPPE_DEV float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
 UPPE_DEV float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// The same sums in one packed instruction (add.rn.f32x2 of sm_100 and later), never contracted with a product
+UPPE_DEV float2 padd(float2 a, float2 b) {
+    float2 r;
+    asm("{\n.reg .b64 x, y, z;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nadd.rn.f32x2 z, x, y;\nmov.b64 {%0, %1}, z;\n}\n"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+UPPE_DEV float2 psub(float2 a, float2 b) {
+    float2 r;
+    asm("{\n.reg .b64 x, y, z;\nmov.b64 x, {%2, %3};\nmov.b64 y, {%4, %5};\nsub.rn.f32x2 z, x, y;\nmov.b64 {%0, %1}, z;\n}\n"
+        : "=f"(r.x), "=f"(r.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
 UPPE_DEV float2 cmul(float2 a, float2 b) { return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x); }
 // The same product with its roundings spelled out: the same bits whatever code surrounds it
 UPPE_DEV float2 cmul_fixed(float2 a, float2 b) {

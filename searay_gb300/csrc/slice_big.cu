@@ -7,8 +7,9 @@
 //                of the tile, the pointwise work of the pass (RK stage, propagator phase, i kz, the
 //                adjoint factors), and/or the inverse column FFT.
 //
-// Both use the register-resident line transforms of slice_reg.cuh (16 values per thread, a 16-point
-// DFT in registers, the line's R = N/16 threads exchange through shared memory).  In the column
+// Both use the line transforms of slice_line.cuh (16 values per thread, a 16-point DFT in registers, the
+// line's R = N/16 threads exchange through shared memory); between the inverse column and row transforms
+// the slice lies in memory with re and im exchanged.  In the column
 // pass a warp holds 16 consecutive columns and two line lanes, so its global accesses are 128-byte
 // row segments; a column's lines span several warps and meet at the CTA barrier.
 //
@@ -18,12 +19,26 @@
 // slice passes (uppe_kernels.cu, slice_reg.cuh) hold for every mode.
 #include <math.h>
 
+#include "slice_line.cuh"
 #include "slice_reg.cuh"
+
+size_t big_line_table_len() { return 64 + 128; }
+
+// {W_N^(j a), W_N^(j (a + 1))} at [a / 2][j], j < N / 16, for N = 128 then 256; FP64
+void big_line_tables(float4* host) {
+    for (int N = 128; N <= 256; N *= 2)
+        for (int i = 0; i < 8; ++i)
+            for (int j = 0; j < N / 16; ++j) {
+                const double a = -2.0 * M_PI * (double)(j * 2 * i) / N, b = -2.0 * M_PI * (double)(j * (2 * i + 1)) / N;
+                host[(N == 256 ? 64 : 0) + i * (N / 16) + j] =
+                    make_float4((float)cos(a), (float)sin(a), (float)cos(b), (float)sin(b));
+            }
+}
 
 template <int LN2, bool INV>
 __global__ void __launch_bounds__(256)
     k_rows_big(const float2* src, float2* dst, float scale, int finish, float2* __restrict__ A_out, OpView opv,
-               int N1, const float2* __restrict__ tw, int twLog, int ahead) {
+               int N1, const float4* __restrict__ tw, int ahead) {
     constexpr int N2 = 1 << LN2, R2 = N2 / 16, ROWS = 256 / R2;
     __shared__ float2 xb[8 * 544];
     const int tid = threadIdx.x;
@@ -35,30 +50,30 @@ __global__ void __launch_bounds__(256)
     const int j = tid % R2;
     float2* ex = xb + (tid >> 5) * 544 + ((tid & 31) / R2) * 17 * R2;
     const LineSync<false> sync{0, 0};
-    const TwGlobal twg{tw, twLog};
+    const float4* twl = line_table<LN2>(tw);
     const float2* s = src + row * N2;
     float2* d = dst + row * N2;
     float2 v[16], w[16];
     if constexpr (!INV) {
 #pragma unroll
         for (int m = 0; m < 16; ++m) v[m] = s[j + R2 * m];
-        reg_n2m<R2, LN2, false>(v, w, ex, j, twg, sync);
+        line_n2m<R2>(v, w, ex, j, twl, sync);
 #pragma unroll
         for (int r = 0; r < 16; ++r) d[j + R2 * (r / R2) + 16 * (r % R2)] = cscale(w[r], scale);
     } else {
 #pragma unroll
         for (int r = 0; r < 16; ++r) w[r] = s[j + R2 * (r / R2) + 16 * (r % R2)];
-        reg_m2n<R2, LN2, true>(w, v, ex, j, twg, sync);
+        line_m2n<R2>(w, v, ex, j, twl, sync);
         if (!finish) {
 #pragma unroll
-            for (int m = 0; m < 16; ++m) d[j + R2 * m] = cscale(v[m], scale);
+            for (int m = 0; m < 16; ++m) d[j + R2 * m] = cscale(swp(v[m]), scale);
         } else {
             // finish: A = IFFT2(e^{..} q), E = i kz A at the same point (uppe_kernel.py:250-253)
             const float2 kgw = opv.kg[row / N1];
 #pragma unroll
             for (int m = 0; m < 16; ++m) {
                 const size_t idx = row * N2 + j + R2 * m;
-                const float2 val = cscale(v[m], scale);
+                const float2 val = cscale(swp(v[m]), scale);
                 if (A_out) A_out[idx] = val;
                 d[j + R2 * m] = cmul(op_ikz(op_at(opv, idx, kgw)), val);
             }
@@ -66,15 +81,16 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// The pass kind is a template parameter (one body per kind keeps each kernel's code small).  The
-// adjoint stage kind runs three blocks per multiprocessor (80 registers: more warps hide its operand
-// loads better than the registers it gives up); the forward fused kind keeps 128 registers, two blocks.  In the
-// kinds that update the RK or adjoint state (BC_FUSED, BC_ADJ_STAGE) the pointwise operands of eight
-// points are loaded before any store of those points: the stores could alias the loads as far as
-// the compiler knows, which otherwise serialises every point behind a full memory latency.
-template <int LN1, int LN2, int KIND>
-__global__ void __launch_bounds__(16 << (LN1 - 4), KIND == BC_ADJ_STAGE ? 3 : 2) k_cols_big(BigColArgs a, OpView opv, const float2* __restrict__ tw,
-                                                              int twLog, int ahead) {
+// The pass kind is a template parameter (one body per kind keeps each kernel's code small), and FAST the form of
+// the fused kind for the mixed precision form in a real medium (PropagatorPair, common.cuh).  The fused kind
+// keeps up to 128 registers, two blocks per multiprocessor (699 us per evaluation of 1025 x 256 x 256 with its row
+// passes; three blocks with 80 registers 779 us); the others run three (80 registers: the inverse kind 634
+// against 810 us at two).  In the kinds that update the RK or adjoint state (BC_FUSED, BC_ADJ_STAGE) the
+// pointwise operands of eight points are loaded before any store of those points: the stores could alias
+// the loads as far as the compiler knows, which otherwise serialises every point behind a full memory latency.
+template <int LN1, int LN2, int KIND, bool FAST>
+__global__ void __launch_bounds__(16 << (LN1 - 4), KIND == BC_FUSED ? 2 : 3)
+    k_cols_big(BigColArgs a, OpView opv, const float4* __restrict__ tw, int ahead) {
     constexpr int N1 = 1 << LN1, N2 = 1 << LN2, R1 = N1 / 16, T = 16 * R1, TILES = N2 / 16;
     constexpr int QC = 17 * R1 + 1;
     __shared__ float2 xb[16 * QC];
@@ -85,12 +101,13 @@ __global__ void __launch_bounds__(16 << (LN1 - 4), KIND == BC_ADJ_STAGE ? 3 : 2)
     const size_t base = (size_t)iw * N1 * N2;
     float2* ex = xb + c * QC;
     const LineSync<true> sync{0, T};
-    const TwGlobal twg{tw, twLog};
+    const float4* twl = line_table<LN1>(tw);
     const PhaseArgs p0{a.z0.zhi, a.z0.zlo, a.z0.plain};
     const PhaseArgs p1{a.z1.zhi, a.z1.zlo, a.z1.plain};
     const float cond = (iw < 4) ? 0.f : 1.f;
     const float2 kgw = opv.kg[iw];
     const int mode = a.mode;
+    const bool same_z = p0.zhi == p1.zhi && p0.zlo == p1.zlo;
     float2 v[16], w[16];
     const auto idx_of = [&](int r) {
         const int kx = i + R1 * (r / R1) + 16 * (r % R1);
@@ -120,7 +137,7 @@ __global__ void __launch_bounds__(16 << (LN1 - 4), KIND == BC_ADJ_STAGE ? 3 : 2)
                 if (pb) asm volatile("prefetch.global.L2 [%0];\n" ::"l"(a.qf + idx));
             }
         }
-        reg_n2m<R1, LN1, false>(v, w, ex, i, twg, sync);
+        line_n2m<R1>(v, w, ex, i, twl, sync);
     }
     if constexpr (KIND == BC_FUSED || KIND == BC_ADJ_STAGE) {
         // BC_FUSED: S and the RK stage (spec_update), E of the next evaluation;
@@ -135,7 +152,7 @@ __global__ void __launch_bounds__(16 << (LN1 - 4), KIND == BC_ADJ_STAGE ? 3 : 2)
             for (int j = 0; j < 8; ++j) {
                 const size_t idx = idx_of(h8 + j);
                 K8[j] = opv.K[idx];
-                ki8[j] = opv.ki ? opv.ki[idx] : 0.f;
+                ki8[j] = !FAST && opv.ki ? opv.ki[idx] : 0.f;
                 A8[j] = need_a ? a.qi[idx] : make_float2(0.f, 0.f);
                 B8[j] = need_b ? a.qf[idx] : make_float2(0.f, 0.f);
             }
@@ -149,8 +166,12 @@ __global__ void __launch_bounds__(16 << (LN1 - 4), KIND == BC_ADJ_STAGE ? 3 : 2)
                 o.kzr = opv.envelope ? kgw.x : (K8[j].x - kgw.x) + (K8[j].y - kgw.y);
                 o.kzi = ki8[j];
                 if constexpr (KIND == BC_FUSED) {
-                    const float2 f = propagator_factor(o, p0, -1.f);
-                    const float2 sv = cscale(cmul_i(cmul(f, w[r])), 0.5f / o.kzr);
+                    PropagatorPair pp;
+                    float2 sv;
+                    if constexpr (FAST)
+                        sv = cscale(cmul_i(pp.backward(o, p0, w[r])), 0.5f / o.kzr);
+                    else
+                        sv = cscale(cmul_i(cmul(propagator_factor(o, p0, -1.f), w[r])), 0.5f / o.kzr);
                     float2 qw;
                     if (mode == SPEC_STAGE1) {
                         a.qf[idx] = cadd(A8[j], cscale(sv, a.Cs));
@@ -163,7 +184,10 @@ __global__ void __launch_bounds__(16 << (LN1 - 4), KIND == BC_ADJ_STAGE ? 3 : 2)
                         a.q_out[idx] = qw;
                     }
                     if (a.q_store && mode != SPEC_FINISH) a.q_store[idx] = qw;
-                    w[r] = cmul(op_ikz(o), cmul(propagator_factor(o, p1, 1.f), qw));
+                    if constexpr (FAST)
+                        w[r] = pp.field(o, p1, same_z, qw);
+                    else
+                        w[r] = cmul(op_ikz(o), cmul(propagator_factor(o, p1, 1.f), qw));
                 } else {
                     const float2 mu = cmul(cconj(op_ikz(o)), cmul(cconj(propagator_factor(o, p0, 1.f)),
                                                                   cscale(w[r], 1.0f / (float)(N1 * N2))));
@@ -219,7 +243,9 @@ __global__ void __launch_bounds__(16 << (LN1 - 4), KIND == BC_ADJ_STAGE ? 3 : 2)
     const bool inverse = (KIND == BC_FUSED || KIND == BC_REAL || KIND == BC_ADJ_IN) ||
                          (KIND == BC_ADJ_STAGE && mode == 1);
     if (inverse) {
-        reg_m2n<R1, LN1, true>(w, v, ex, i, twg, sync);
+#pragma unroll
+        for (int r = 0; r < 16; ++r) w[r] = swp(w[r]);
+        line_m2n<R1>(w, v, ex, i, twl, sync);
 #pragma unroll
         for (int m = 0; m < 16; ++m) a.dst[base + (size_t)(i + R1 * m) * N2 + ky] = v[m];
     }
@@ -242,22 +268,22 @@ static cudaError_t rows(UppeHandle* h, const float2* src, float2* dst, float sca
     const OpView opv = uppe_op_view(h);
     if (h->N2 == 256) {
         k_rows_big<8, INV><<<(unsigned)(nrows / 16), 256, 0, h->stream>>>(src, dst, scale, finish, A_out, opv, h->N1,
-                                                                         h->tw, h->twLog, 2 * h->num_sms);
+                                                                         h->tw_line, 2 * h->num_sms);
     } else {
         k_rows_big<7, INV><<<(unsigned)(nrows / 32), 256, 0, h->stream>>>(src, dst, scale, finish, A_out, opv, h->N1,
-                                                                         h->tw, h->twLog, 2 * h->num_sms);
+                                                                         h->tw_line, 2 * h->num_sms);
     }
     return cudaGetLastError();
 }
 
-template <int KIND>
+template <int KIND, bool FAST = false>
 static void cols_kind(UppeHandle* h, const BigColArgs& a, const OpView& opv, unsigned grid) {
     if (h->N1 == 256 && h->N2 == 256)
-        k_cols_big<8, 8, KIND><<<grid, 256, 0, h->stream>>>(a, opv, h->tw, h->twLog, 2 * h->num_sms);
+        k_cols_big<8, 8, KIND, FAST><<<grid, 256, 0, h->stream>>>(a, opv, h->tw_line, 2 * h->num_sms);
     else if (h->N1 == 256)
-        k_cols_big<8, 7, KIND><<<grid, 256, 0, h->stream>>>(a, opv, h->tw, h->twLog, 2 * h->num_sms);
+        k_cols_big<8, 7, KIND, FAST><<<grid, 256, 0, h->stream>>>(a, opv, h->tw_line, 2 * h->num_sms);
     else
-        k_cols_big<7, 8, KIND><<<grid, 128, 0, h->stream>>>(a, opv, h->tw, h->twLog, 2 * h->num_sms);
+        k_cols_big<7, 8, KIND, FAST><<<grid, 128, 0, h->stream>>>(a, opv, h->tw_line, 2 * h->num_sms);
 }
 
 // Column passes of the slices [0, nslices) (every slice when nslices < 0).
@@ -266,7 +292,12 @@ static cudaError_t cols(UppeHandle* h, const BigColArgs& a, int nslices = -1) {
     const OpView opv = uppe_op_view(h);
     const unsigned grid = (unsigned)((nslices < 0 ? h->N0 : nslices) * (h->N2 / 16));
     switch (a.kind) {
-        case BC_FUSED: cols_kind<BC_FUSED>(h, a, opv, grid); break;
+        case BC_FUSED:
+            if (h->cfg.precision == UPPE_PREC_MIXED && !h->complex_medium)
+                cols_kind<BC_FUSED, true>(h, a, opv, grid);
+            else
+                cols_kind<BC_FUSED>(h, a, opv, grid);
+            break;
         case BC_SPEC: cols_kind<BC_SPEC>(h, a, opv, grid); break;
         case BC_REAL: cols_kind<BC_REAL>(h, a, opv, grid); break;
         case BC_ADJ_IN: cols_kind<BC_ADJ_IN>(h, a, opv, grid); break;

@@ -16,13 +16,14 @@
 // HBM traffic per point: J 8, K 8, qi and/or qf 8-16, qf or qi 8, E 8: 40-48 bytes.
 //
 // 512 threads and about 133 KB of shared memory per CTA: one CTA per multiprocessor, a cluster on 8
-// multiprocessors.  Measured on 1025 x 256 x 256 it takes 1.86 ms per evaluation against 0.90 ms
+// multiprocessors.  Measured on 1025 x 256 x 256 it took 1.86 ms per evaluation against 0.90 ms
 // for the three passes (one CTA per multiprocessor leaves each phase's memory latency exposed), so
 // it is selected only on request (SEARAY_UPPE_CLUSTER=1); it gives the three-pass results bit for bit.
 // Every CTA of a cluster runs the same barrier sequence; there are no waits on flags.  The slices without current (w >= nl_cut_off, J = 0 from the NL filter) skip the load and
 // the forward row transform and run the rest on zeros (S = 0 exactly).
 #include <cooperative_groups.h>
 
+#include "slice_line.cuh"
 #include "slice_reg.cuh"
 
 namespace cg = cooperative_groups;
@@ -42,7 +43,7 @@ __device__ __forceinline__ void sc_cluster_arrive() { asm volatile("barrier.clus
 __device__ __forceinline__ void sc_cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory"); }
 
 __global__ void __cluster_dims__(SC_CL, 1, 1) __launch_bounds__(SC_THREADS, 1)
-    k_slice_cluster(BigColArgs a, OpView opv, const float2* __restrict__ tw, int twLog, int nfwd, float inv_s,
+    k_slice_cluster(BigColArgs a, OpView opv, const float4* __restrict__ tw, int nfwd, float inv_s,
                     float2* __restrict__ E_out) {
     extern __shared__ float2 scm[];
     float2* T = scm;
@@ -52,7 +53,7 @@ __global__ void __cluster_dims__(SC_CL, 1, 1) __launch_bounds__(SC_THREADS, 1)
     const int iw = blockIdx.x / SC_CL;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const size_t base = (size_t)iw * SC_N * SC_N;
-    const TwGlobal twg{tw, twLog};
+    const float4* twl = line_table<8>(tw);
     float2 v[16], w[16];
 
     // ---- 1. rows x = 32 r + xl: forward transform along y ----
@@ -63,7 +64,7 @@ __global__ void __cluster_dims__(SC_CL, 1, 1) __launch_bounds__(SC_THREADS, 1)
         const float2* s = a.src + base + (size_t)(SC_ROWS * r + xl) * SC_N + j;
 #pragma unroll
         for (int m = 0; m < 16; ++m) v[m] = s[16 * m];
-        reg_n2m<16, 8, false>(v, w, exr, j, twg, rsync);  // w[b] = X[x][j + 16 b]
+        line_n2m<16>(v, w, exr, j, twl, rsync);  // w[b] = X[x][j + 16 b]
     } else {
 #pragma unroll
         for (int b = 0; b < 16; ++b) w[b] = make_float2(0.f, 0.f);
@@ -85,7 +86,7 @@ __global__ void __cluster_dims__(SC_CL, 1, 1) __launch_bounds__(SC_THREADS, 1)
     sc_cluster_arrive();  // this CTA's reads of the cluster's T are done
     float2* exc = EX + kyl * (17 * 16 + 1);
     const LineSync<true> csync{1 + tile, 256};
-    reg_n2m<16, 8, false>(v, w, exc, i, twg, csync);  // w[q] at kx = i + 16 q
+    line_n2m<16>(v, w, exc, i, twl, csync);  // w[q] at kx = i + 16 q
     {
         const PhaseArgs p0{a.z0.zhi, a.z0.zlo, a.z0.plain};
         const PhaseArgs p1{a.z1.zhi, a.z1.zlo, a.z1.plain};
@@ -135,7 +136,9 @@ __global__ void __cluster_dims__(SC_CL, 1, 1) __launch_bounds__(SC_THREADS, 1)
             }
         }
     }
-    reg_m2n<16, 8, true>(w, v, exc, i, twg, csync);  // v[m] at x = i + 16 m
+#pragma unroll
+    for (int q = 0; q < 16; ++q) w[q] = swp(w[q]);
+    line_m2n<16>(w, v, exc, i, twl, csync);  // v[m] at x = i + 16 m, re and im exchanged from here on
     sc_cluster_wait();  // every CTA has read this CTA's T: overwrite it with the columns
 #pragma unroll
     for (int m = 0; m < 16; ++m) T[kyl * SC_PT + i + 16 * m] = v[m];
@@ -151,10 +154,10 @@ __global__ void __cluster_dims__(SC_CL, 1, 1) __launch_bounds__(SC_THREADS, 1)
         w[b] = Tq[(kyb % SC_ROWS) * SC_PT + x];
     }
     sc_cluster_arrive();  // this CTA's reads of the cluster's T are done
-    reg_m2n<16, 8, true>(w, v, exr, j, twg, rsync);
+    line_m2n<16>(w, v, exr, j, twl, rsync);
     float2* d = E_out + base + (size_t)x * SC_N + j;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) d[16 * m] = cscale(v[m], inv_s);
+    for (int m = 0; m < 16; ++m) d[16 * m] = cscale(swp(v[m]), inv_s);
     sc_cluster_wait();  // no CTA leaves while another may still read its shared memory
 }
 
@@ -196,7 +199,7 @@ cudaError_t launch_fused_cluster(UppeHandle* h, const BigColArgs& a, int nfwd, i
     if (!cluster_slice_supported(h->N1, h->N2) || !cluster_slice_ready()) return cudaErrorNotSupported;
     h->launches++;
     const OpView opv = uppe_op_view(h);
-    k_slice_cluster<<<(unsigned)(nall * SC_CL), SC_THREADS, SC_SMEM, h->stream>>>(a, opv, h->tw, h->twLog, nfwd,
+    k_slice_cluster<<<(unsigned)(nall * SC_CL), SC_THREADS, SC_SMEM, h->stream>>>(a, opv, h->tw_line, nfwd,
                                                                                    1.0f / (float)h->S, h->E);
     return cudaGetLastError();
 }

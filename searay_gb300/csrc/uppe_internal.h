@@ -69,6 +69,7 @@ struct UppeHandle {
     int complex_medium;
     float* ng;
     float2* tw;
+    float4* tw_line; // twiddle tables of the big slices' line transforms (slice_big.cu), or NULL
     float2* tw_reg;  // twiddle tables of the register-resident time pass (timepass_reg.cu), or NULL
     float2* tscr;    // its parking scratch for ionizing columns ([S][2 (M + 1)]), or NULL
     int* adj_live;   // register-resident adjoint time pass: count + column groups left to k_time_adj, or NULL
@@ -192,6 +193,8 @@ cudaError_t launch_adj_fused_big(UppeHandle* h, int mode, const float2* g, float
 
 // ---- Cartesian slices of 128 x 256, 256 x 128, 256 x 256 (slice_big.cu): row + column passes ----
 bool big_slice_supported(int N1, int N2);
+size_t big_line_table_len();
+void big_line_tables(float4* host);
 struct BigColArgs;
 // the fused tail of 256 x 256 slices in one launch (a cluster of 8 CTAs per slice); returns
 // cudaErrorNotSupported where the cluster form cannot run
