@@ -1,5 +1,5 @@
-"""The fused slice pass in its two forms: the one for a real medium in the mixed precision form (one phasor for both
-propagator factors where they are at the same z, no Im kz) and the general one (searay_gb300/csrc/slice_reg.cuh).
+"""The fused slice passes in their two forms: the one for a real medium in the mixed precision form (one phasor for both
+propagator factors where they are at the same z, no Im kz) and the general one (searay_gb300/csrc/slice_reg.cuh, slice_big.cu).
 
 The same volume is stepped with a real medium and with one that absorbs in the last frequency bin only,
 which selects the general form.  That bin lies above the nonlinear band and holds no field, so every
@@ -31,7 +31,8 @@ class LastBinAbsorbs:
 
 
 @pytest.mark.parametrize("adaptive", [False, True], ids=["fixed", "adaptive"])
-@pytest.mark.parametrize("shape", [(65, 16, 16), (65, 16, 128), (129, 64, 32), (65, 128, 128)],
+@pytest.mark.parametrize("shape", [(65, 16, 16), (65, 16, 128), (129, 64, 32), (65, 128, 128), (33, 256, 128),
+                                   (33, 128, 256), (33, 256, 256)],
                          ids=lambda s: "x".join(map(str, s)))
 def test_real_and_general_medium(shape, adaptive):
     import torch
