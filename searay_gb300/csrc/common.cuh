@@ -63,6 +63,8 @@ UPPE_DEV float2 cmul_conj_fixed(float2 f, float2 a) {
     return make_float2(fmaf(f.x, a.x, __fmul_rn(f.y, a.y)), fmaf(-f.y, a.x, __fmul_rn(f.x, a.y)));
 }
 UPPE_DEV float2 cscale(float2 a, float s) { return make_float2(a.x * s, a.y * s); }
+// a + b, never contracted with a product
+UPPE_DEV float2 cadd_fixed(float2 a, float2 b) { return make_float2(__fadd_rn(a.x, b.x), __fadd_rn(a.y, b.y)); }
 // a + s b, each component one fused multiply-add whatever surrounds it
 UPPE_DEV float2 caxpy(float2 a, float2 b, float s) { return make_float2(fmaf(b.x, s, a.x), fmaf(b.y, s, a.y)); }
 UPPE_DEV float2 cconj(float2 a) { return make_float2(a.x, -a.y); }

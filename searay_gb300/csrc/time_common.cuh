@@ -17,6 +17,7 @@ struct TimeParams {
     float c2[6];           // series form: log2(e) * c_i, polynomial in L = ln(Em)
     float em_min;          // below this Em the rate is below FP32's smallest normal (taken as 0)
     int wcut, wwid, plain;
+    float inv_wwid;        // 1 / wwid where that is exact (a power of two), else 0
     int cut_on, cut_off;   // NL filter: J is kept for cut_on <= k < cut_off (uppe_kernel.py:122-125)
     // rotational Raman: transitions in pairs, 20 float4 per pair (constants and powers of h^2) and
     // the phasor table p0[pair][segment] (raman_pass)
@@ -31,51 +32,72 @@ struct TimeParams {
 
 #define UPPE_LN2 0.69314718055994530942f
 
-// Ionization rate in simulation units from the field in simulation units.
-__device__ __forceinline__ float ion_rate(const TimeParams& tp, float e) {
+// 1 / x correctly rounded, for normal |x| below 2^126: one Newton step on the hardware's approximation with the
+// residual taken by FMA (P. W. Markstein, IBM J. Res. Dev. 34 (1990) 111).  Equal to __frcp_rn for every
+// significand there, without its branch for the other cases, which keeps the evaluations around it apart.
+__device__ __forceinline__ float rcp_normal(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return fmaf(y, fmaf(-x, y, 1.f), y);
+}
+
+// Ionization rate in simulation units from the field in simulation units, by the closed form (EXPLICIT) or the
+// series.  No branch per sample (the zero below em_min is selected), so that the evaluations of a thread's
+// samples overlap.
+template <bool EXPLICIT>
+__device__ __forceinline__ float ion_rate_form(const TimeParams& tp, float e) {
     const float em = fmaf(tp.fconv, fabsf(e), tp.cutoff);
-    if (em < tp.em_min) return 0.f;
     const float l2 = __log2f(em);
-    if (tp.rate_form == UPPE_RATE_EXPLICIT) {
-        return exp2f(fmaf(tp.ypow, l2, fmaf(tp.yexp, __frcp_rn(em), tp.y0)));
+    float r;
+    if constexpr (EXPLICIT) {
+        r = exp2f(fmaf(tp.ypow, l2, fmaf(tp.yexp, rcp_normal(em), tp.y0)));
+    } else {
+        const float L = l2 * UPPE_LN2;
+        float p = tp.c2[5];
+        p = fmaf(p, L, tp.c2[4]);
+        p = fmaf(p, L, tp.c2[3]);
+        p = fmaf(p, L, tp.c2[2]);
+        p = fmaf(p, L, tp.c2[1]);
+        p = fmaf(p, L, tp.c2[0]);
+        r = exp2f(tp.lrc2 + p);
     }
-    const float L = l2 * UPPE_LN2;
-    float p = tp.c2[5];
-    p = fmaf(p, L, tp.c2[4]);
-    p = fmaf(p, L, tp.c2[3]);
-    p = fmaf(p, L, tp.c2[2]);
-    p = fmaf(p, L, tp.c2[1]);
-    p = fmaf(p, L, tp.c2[0]);
-    return exp2f(tp.lrc2 + p);
+    return em < tp.em_min ? 0.f : r;
+}
+__device__ __forceinline__ float ion_rate(const TimeParams& tp, float e) {
+    return tp.rate_form == UPPE_RATE_EXPLICIT ? ion_rate_form<true>(tp, e) : ion_rate_form<false>(tp, e);
 }
 
 __device__ __forceinline__ float smooth5(float q) { return q * q * q * (10.f - 15.f * q + 6.f * q * q); }
 
-__device__ __forceinline__ float soft_window(int i, int Ni, int cut, int wid) {
+// SoftTimeWindow (fft.cl:331-355) at sample i of Ni.  The distance into a ramp over its width: for a power of two (the
+// reference's 64) the product with the exact reciprocal, which the division equals.
+__device__ __forceinline__ float soft_window(const TimeParams& tp, int i, int Ni) {
+    const int cut = tp.wcut, wid = tp.wwid;
+    const auto ramp = [&](int d) {
+        return smooth5(tp.inv_wwid != 0.f ? (float)d * tp.inv_wwid : (float)d / (float)wid);
+    };
     float f = 1.f;
     if (i < cut || i > Ni - cut - 1) f = 0.f;
-    if (i >= cut && i < cut + wid) f *= smooth5((float)(i - cut) / (float)wid);
-    if (i <= Ni - cut - 1 && i > Ni - cut - wid - 1) f *= smooth5((float)(Ni - cut - 1 - i) / (float)wid);
+    if (i >= cut && i < cut + wid) f *= ramp(i - cut);
+    if (i <= Ni - cut - 1 && i > Ni - cut - wid - 1) f *= ramp(Ni - cut - 1 - i);
     return f;
 }
 
 // 1 - exp(-S) for S >= 0: the Taylor series of -expm1(-S) through S^8 (truncation below 1e-11
 // relative) for S < 1/4, where 1 - exp(-S) would cancel, and 1 - expf(-S) above.
+// Both are evaluated and one is selected: no branch per sample.
 __device__ __forceinline__ float one_minus_exp_neg(float S) {
-    if (S == 0.f) return 0.f;
-    if (S < 0.25f) {
-        const float x = -S;
-        float p = 1.f / 40320.f;
-        p = fmaf(p, x, 1.f / 5040.f);
-        p = fmaf(p, x, 1.f / 720.f);
-        p = fmaf(p, x, 1.f / 120.f);
-        p = fmaf(p, x, 1.f / 24.f);
-        p = fmaf(p, x, 1.f / 6.f);
-        p = fmaf(p, x, 0.5f);
-        p = fmaf(p, x, 1.f);
-        return -x * p;
-    }
-    return 1.f - expf(-S);
+    const float x = -S;
+    float p = 1.f / 40320.f;
+    p = fmaf(p, x, 1.f / 5040.f);
+    p = fmaf(p, x, 1.f / 720.f);
+    p = fmaf(p, x, 1.f / 120.f);
+    p = fmaf(p, x, 1.f / 24.f);
+    p = fmaf(p, x, 1.f / 6.f);
+    p = fmaf(p, x, 0.5f);
+    p = fmaf(p, x, 1.f);
+    const float far = 1.f - expf(-S);
+    return S < 0.25f ? -x * p : far;
 }
 
 __device__ __forceinline__ void acc_add(ffloat& s, float p, int plain) {

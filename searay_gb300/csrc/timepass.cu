@@ -145,12 +145,12 @@ __global__ void __launch_bounds__(ET == 16 ? 256 : 512,
             const float2 zv = Zp[sw(m) * C + c];
             const int t = 2 * m + 1;
             const float r1 = (t == Nt - 1) ? 0.f : ion_rate(tp, zv.y * inv);
-            const float p1 = tp.hdt * (r1 + rn);
-            if (t <= Nt - 2 && p1 != 0.f) acc_add(part, p1, tp.plain);
+            const float p1 = __fmul_rn(tp.hdt, r1 + rn);
+            acc_add(part, p1, tp.plain);  // (p1 = 0 at the last sample)
             const float r0 = ion_rate(tp, zv.x * inv);
-            const float p0 = tp.hdt * (r0 + r1);
-            if (p0 != 0.f) acc_add(part, p0, tp.plain);
-            live = live || r0 != 0.f || r1 != 0.f;
+            const float p0 = __fmul_rn(tp.hdt, r0 + r1);
+            acc_add(part, p0, tp.plain);
+            live = live | (r0 != 0.f) | (r1 != 0.f);
             rn = r0;
             Zj[sw(m) * C + c] = make_float2(r0, r1);  // this thread's own slot, reused below
         }
@@ -211,13 +211,13 @@ __global__ void __launch_bounds__(ET == 16 ? 256 : 512,
             if (dens) {
                 const float2 rr = Zj[sw(m) * C + c];
                 const int t = 2 * m + 1;
-                if (t <= Nt - 2) acc_add(Sacc, tp.hdt * (rr.y + rn), tp.plain);
+                acc_add(Sacc, tp.hdt * (rr.y + rn), tp.plain);
                 ne1 = ngc * one_minus_exp_neg(ff_value(Sacc));
-                if (t < wlo || t > whi) ne1 *= soft_window(t, Nt, tp.wcut, tp.wwid);
+                if (t < wlo || t > whi) ne1 *= soft_window(tp, t, Nt);
                 acc_add(Sacc, tp.hdt * (rr.x + rr.y), tp.plain);
                 rn = rr.x;
                 ne0 = ngc * one_minus_exp_neg(ff_value(Sacc));
-                if (t - 1 < wlo || t - 1 > whi) ne0 *= soft_window(t - 1, Nt, tp.wcut, tp.wwid);
+                if (t - 1 < wlo || t - 1 > whi) ne0 *= soft_window(tp, t - 1, Nt);
             }
             float chi1 = kerr * e1 * e1, chi0 = kerr * e0 * e0;
             if constexpr (RAMAN != 0) {  // the Raman chi comes first in the reference's sum (uppe_kernel.py:173-179)
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(ET == 16 ? 256 : 512,
             const float wk = wv[k];
             float2 J = cmul_mi(cscale(P, wk));  // -i w P
             if (two) {  // Jpl / (damping - i w) = Jpl (damping + i w) / (damping^2 + w^2)
-                const float rden = __frcp_rn(fmaf(wk, wk, tp.damping * tp.damping));
+                const float rden = rcp_normal(fmaf(wk, wk, tp.damping * tp.damping));
                 J = cadd(J, cscale(cmul(Q, make_float2(tp.damping, wk)), rden));
             }
             if (tp.atc)
@@ -320,6 +320,7 @@ TimeParams uppe_time_params(const UppeHandle* h) {
     tp.cut_on = c.nl_cut_on;
     tp.cut_off = c.nl_cut_off;
     tp.wwid = c.window_width;
+    tp.inv_wwid = (c.window_width > 0 && (c.window_width & (c.window_width - 1)) == 0) ? 1.f / (float)c.window_width : 0.f;
     tp.plain = (c.precision == UPPE_PREC_FP32);
     tp.rot_pairs = h->rot_pairs;
     tp.rot_tab = reinterpret_cast<const float4*>(h->rot);
@@ -677,8 +678,8 @@ __global__ void __launch_bounds__(LOGM > 0 ? 256 : 512, RAMAN ? 1 : (LOGM > 0 ? 
             for (int j = 0; j < MPS; ++j) {
                 const int m = m0 + j;
                 const float2 e2 = Ze[sw(m) * C + c], l2 = Zl[sw(m) * C + c], s2 = Zn[sw(m) * C + c];
-                const float a0 = ngc * soft_window(2 * m, Nt, tp.wcut, tp.wwid) * expf(-s2.x);
-                const float a1 = ngc * soft_window(2 * m + 1, Nt, tp.wcut, tp.wwid) * expf(-s2.y);
+                const float a0 = ngc * soft_window(tp, 2 * m, Nt) * expf(-s2.x);
+                const float a1 = ngc * soft_window(tp, 2 * m + 1, Nt) * expf(-s2.y);
                 acc_add(part, l2.x * e2.x * inv * a0, tp.plain);
                 acc_add(part, l2.y * e2.y * inv * a1, tp.plain);
             }
@@ -711,7 +712,7 @@ __global__ void __launch_bounds__(LOGM > 0 ? 256 : 512, RAMAN ? 1 : (LOGM > 0 ? 
                     if (ion) {
                         const float gl = h ? l2.y : l2.x;
                         const float Sv = h ? s2.y : s2.x;
-                        const float wv_t = soft_window(t, Nt, tp.wcut, tp.wwid);
+                        const float wv_t = soft_window(tp, t, Nt);
                         const float ne = ngc * one_minus_exp_neg(Sv) * wv_t;
                         const float a = ngc * wv_t * expf(-Sv);
                         g = fmaf(ne, gl, g);

@@ -24,6 +24,14 @@
 // order) and then the P part of J (frequency order) in a global scratch array, column-contiguous
 // (coalesced), until the Jpl transform is done.
 //
+// An ionizing column is a long chain for its warp, and a block waits for its slowest.  Measured by clock64 stamps
+// at M = 1024 (cycles): rates 14-20k, two scans 4k + 5k, densities 33k, unpacking with the plasma current 10k of
+// 100k.  What held it up were branches around every sample's rate, exponential and reciprocal (the samples of a
+// lane could not overlap), the soft window's divisions in the end lanes at every step of the scan, and loads of the
+// parked current each behind the store before it.  Branch-free samples (time_common.cuh), the window
+// applied once on neighbouring samples and the parked current asked eight bins ahead: 57 -> 32 us a pass on
+// 1025 x 64 to 512 ionizing columns, 28 -> 17 us on 257 x 512; 68.7 -> 58.6 us on 513 x 128 x 128.
+//
 // Block: NC columns x TC lanes = 256 threads.  The half spectra of the NC columns are staged into
 // shared memory with 8-byte cp.async (rows of NC columns: coalesced), one buffer of LD complex
 // values per column that then serves the exchanges, the density scan and the output staging; J is
@@ -88,30 +96,34 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
     if (live) {
         // rates in natural order (padded positions)
         __syncwarp();  // exchange reads of buf are done
+        const auto rates = [&](auto rate) {
 #pragma unroll
-        for (int r = 0; r < R1; ++r) {
-            const int m = G::tm(t, r);
-            const float2 z = v[r];
-            const float r0 = ion_rate(tp, z.x * inv);
-            const float r1 = (2 * m + 1 == G::NT - 1) ? 0.f : ion_rate(tp, z.y * inv);
-            buf[tr_pad<G::LSEG>(m)] = make_float2(r0, r1);
-        }
+            for (int r = 0; r < R1; ++r) {
+                const int m = G::tm(t, r);
+                const float2 z = v[r];
+                const float r0 = rate(z.x * inv);
+                const float r1 = (2 * m + 1 == G::NT - 1) ? 0.f : rate(z.y * inv);
+                buf[tr_pad<G::LSEG>(m)] = make_float2(r0, r1);
+            }
+        };
+        if (tp.rate_form == UPPE_RATE_EXPLICIT)
+            rates([&](float e) { return ion_rate_form<true>(tp, e); });
+        else
+            rates([&](float e) { return ion_rate_form<false>(tp, e); });
         __syncwarp();
         // density: lane t scans the pairs [t SEG, (t+1) SEG) from high to low time
         const int mb = t * G::SEG;
         const float r_next = (t < TC - 1) ? buf[tr_pad<G::LSEG>(mb + G::SEG)].x : 0.f;
+        // (the last pair's odd increment is 0, as its rates are, and adding a zero increment leaves a
+        // float-float sum as it is: no conditions in the scans)
         ffloat part = {0.f, 0.f};
         {
             float rn = r_next;
+#pragma unroll 4
             for (int i = G::SEG - 1; i >= 0; --i) {
-                const int m = mb + i;
-                const float2 rr = buf[tr_pad<G::LSEG>(m)];
-                if (2 * m + 1 <= G::NT - 2) {
-                    const float p1 = tp.hdt * (rr.y + rn);
-                    if (p1 != 0.f) acc_add(part, p1, tp.plain);
-                }
-                const float p0 = tp.hdt * (rr.x + rr.y);
-                if (p0 != 0.f) acc_add(part, p0, tp.plain);
+                const float2 rr = buf[tr_pad<G::LSEG>(mb + i)];
+                acc_add(part, __fmul_rn(tp.hdt, rr.y + rn), tp.plain);
+                acc_add(part, __fmul_rn(tp.hdt, rr.x + rr.y), tp.plain);
                 rn = rr.x;
             }
         }
@@ -134,20 +146,30 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
         if (t == TC - 1) Sacc = ffloat{0.f, 0.f};
         __syncwarp();  // every lane has read its neighbour's first rate
         {
-            const int wlo = tp.wcut + tp.wwid, whi = G::NT - tp.wcut - tp.wwid - 1;  // window is 1 on [wlo, whi]
             float rn = r_next;
+#pragma unroll 4
             for (int i = G::SEG - 1; i >= 0; --i) {
-                const int m = mb + i;
-                const float2 rr = buf[tr_pad<G::LSEG>(m)];
-                const int t1 = 2 * m + 1;
-                if (t1 <= G::NT - 2) acc_add(Sacc, tp.hdt * (rr.y + rn), tp.plain);
-                float ne1 = ngc * one_minus_exp_neg(ff_value(Sacc));
-                if (t1 < wlo || t1 > whi) ne1 *= soft_window(t1, G::NT, tp.wcut, tp.wwid);
-                acc_add(Sacc, tp.hdt * (rr.x + rr.y), tp.plain);
-                float ne0 = ngc * one_minus_exp_neg(ff_value(Sacc));
-                if (t1 - 1 < wlo || t1 - 1 > whi) ne0 *= soft_window(t1 - 1, G::NT, tp.wcut, tp.wwid);
-                rn = rr.x;
-                buf[tr_pad<G::LSEG>(m)] = make_float2(ne0, ne1);
+                float2& rr = buf[tr_pad<G::LSEG>(mb + i)];
+                const float2 r = rr;
+                acc_add(Sacc, tp.hdt * (r.y + rn), tp.plain);
+                const float ne1 = ngc * one_minus_exp_neg(ff_value(Sacc));
+                acc_add(Sacc, tp.hdt * (r.x + r.y), tp.plain);
+                rr = make_float2(ngc * one_minus_exp_neg(ff_value(Sacc)), ne1);
+                rn = r.x;
+            }
+        }
+        __syncwarp();
+        // the soft window on the samples where it is not 1 (wlo at each end), lanes on neighbouring pairs: in the
+        // scan, the end lanes' divisions held the warp up at every step
+        const int wlo = tp.wcut + tp.wwid;
+#pragma unroll 1
+        for (int m = t; m < M && 2 * m < wlo; m += TC) {
+#pragma unroll 1
+            for (int end = 0; end < 2; ++end) {
+                const int me = end ? M - 1 - m : m;
+                float2& ne = buf[tr_pad<G::LSEG>(me)];
+                ne.x *= soft_window(tp, 2 * me, G::NT);
+                ne.y *= soft_window(tp, 2 * me + 1, G::NT);
             }
         }
         __syncwarp();
@@ -189,12 +211,15 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
         tr_forward<LOGM>(v, buf, twF, t);
         __syncwarp();
         const float damp = tp.damping;
-        tr_unpack<LOGM>(v, twP, t, lane, [&](int k, float2 Q) {
-            const float wk = __ldg(&wv[k]);
-            const float rden = __frcp_rn(fmaf(wk, wk, damp * damp));
-            const float2 q = cscale(cmul(Q, make_float2(damp, wk)), rden);
-            buf[k] = kept(k) ? cadd(parkJ[k], q) : make_float2(0.f, 0.f);
-        });
+        tr_unpack_with<LOGM>(
+            v, twP, t, lane,
+            [&](int k, float2 Q, float2 PJ) {
+                const float wk = __ldg(&wv[k]);
+                const float rden = rcp_normal(fmaf(wk, wk, damp * damp));
+                const float2 q = cscale(cmul(Q, make_float2(damp, wk)), rden);
+                buf[k] = kept(k) ? cadd_fixed(PJ, q) : make_float2(0.f, 0.f);
+            },
+            [&](int k) { return parkJ[k]; });
     }
 
     // ---- write J back: rows of NC columns ----

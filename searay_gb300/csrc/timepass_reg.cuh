@@ -193,6 +193,36 @@ UPPE_DEV void tr_unpack(const float2 (&v)[TReg<LOGM>::R1], const float2* __restr
 }
 
 
+// tr_unpack with a value from memory for every bin: emit(k, X[k], with(k)), with asked eight bins before the first
+// of them is emitted (the stores of emit would hold back each load in turn).
+template <int LOGM, class Emit, class With>
+UPPE_DEV void tr_unpack_with(const float2 (&v)[TReg<LOGM>::R1], const float2* __restrict__ twP, int t, int lane,
+                             Emit emit, With with) {
+    using G = TReg<LOGM>;
+    const int partner = (lane & ~(G::TC - 1)) | ((G::TC - t) & (G::TC - 1));
+#pragma unroll
+    for (int a8 = 0; a8 < G::R1; a8 += 8) {
+        float2 m[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) m[i] = with(t + G::TC * (a8 + i));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int a = a8 + i;
+            const float2 send = v[G::R1 - 1 - a];
+            float2 got;
+            got.x = __shfl_sync(0xffffffffu, send.x, partner);
+            got.y = __shfl_sync(0xffffffffu, send.y, partner);
+            if (t == 0) got = v[(G::R1 - a) & (G::R1 - 1)];
+            const float2 twk = __ldg(&twP[a * G::TC + t]);
+            const float2 Zb = cconj(got);
+            const float2 s = cadd(v[a], Zb);
+            const float2 d = cmul(twk, csub(v[a], Zb));
+            emit(t + G::TC * a, cscale(csub(s, cmul_i(d)), 0.5f), m[i]);
+        }
+    }
+    if (t == 0) emit(G::M, make_float2(v[0].x - v[0].y, 0.f), with(G::M));
+}
+
 // Even/odd packing of the half spectrum X(k), k in [0, M] (xk(k) gives X[k]; its imaginary parts
 // at k = 0 and M do not enter irfft), into the F layout, then the inverse transform into the T
 // layout: v[j TC + c] = z[t + TC j + R1 c] with z[m] = Nt (x(2m) + i x(2m+1)) of x = irfft(X).
