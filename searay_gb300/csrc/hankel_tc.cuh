@@ -47,6 +47,44 @@ __device__ __forceinline__ void tc_store_split(uint8_t* __restrict__ Atc, int nw
     *reinterpret_cast<__nv_bfloat16*>(tile + TC_TILE_BYTES + oim) = il;
 }
 
+// The bf16 halves of a pair of values as two 32-bit words, the first value in the low half.
+__device__ __forceinline__ void split_bf16x2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
+    const __nv_bfloat162 l = __floats2bfloat162_rn(a - __low2float(h), b - __high2float(h));
+    hi = *reinterpret_cast<const uint32_t*>(&h);
+    lo = *reinterpret_cast<const uint32_t*>(&l);
+}
+
+// tc_store_split for neighbouring lanes k, k ^ 1 of one w (both active): the even lane stores the real row's two
+// values, the odd lane the imaginary row's, 4 bytes a store instead of 2.  (In the spectral update and the operand pre-pass,
+// whose eight neighbouring lanes already fill a 16-byte row, the exchange cost more than the stores saved.)
+__device__ __forceinline__ void tc_store_pair(uint8_t* __restrict__ Atc, int nwt, int nkt, int m, int w, int k,
+                                              float2 v) {
+    const bool odd = k & 1;
+    const float got = __shfl_xor_sync(3u << (threadIdx.x & 30), odd ? v.x : v.y, 1);
+    uint32_t hi, lo;
+    split_bf16x2(odd ? got : v.x, odd ? v.y : got, hi, lo);
+    const unsigned uw = (unsigned)w, uk = (unsigned)k & ~1u;
+    uint8_t* tile = Atc + (((size_t)m * nwt + uw / TC_W) * nkt + uk / TC_K) * (size_t)(2 * TC_TILE_BYTES);
+    const uint32_t o = core_off(2 * (int)(uw % TC_W) + (odd ? 1 : 0), (int)(uk % TC_K));
+    *reinterpret_cast<uint32_t*>(tile + o) = hi;
+    *reinterpret_cast<uint32_t*>(tile + TC_TILE_BYTES + o) = lo;
+}
+
+// Eight columns k .. k + 7 (k a multiple of 8) of one row (part 0: re, 1: im of w) of azimuthal mode 0: x[0 .. 8)
+// as one 16-byte store to each tile.
+__device__ __forceinline__ void tc_store_row8(uint8_t* __restrict__ Atc, int nkt, int w, int part, int k,
+                                              const float (&x)[8]) {
+    uint32_t h[4], l[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) split_bf16x2(x[2 * i], x[2 * i + 1], h[i], l[i]);
+    const unsigned uw = (unsigned)w, uk = (unsigned)k;
+    uint8_t* tile = Atc + ((size_t)(uw / TC_W) * nkt + uk / TC_K) * (size_t)(2 * TC_TILE_BYTES);
+    const uint32_t o = core_off(2 * (int)(uw % TC_W) + part, (int)(uk % TC_K));
+    *reinterpret_cast<uint4*>(tile + o) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4*>(tile + TC_TILE_BYTES + o) = make_uint4(l[0], l[1], l[2], l[3]);
+}
+
 // The next inverse transform's operand, written by the spectral update of the stage before it:
 // Atc NULL when not asked.
 struct TcNext {

@@ -261,7 +261,9 @@ __global__ void __launch_bounds__(ET == 16 ? 256 : 512,
                 const float rden = rcp_normal(fmaf(wk, wk, tp.damping * tp.damping));
                 J = cadd(J, cscale(cmul(Q, make_float2(tp.damping, wk)), rden));
             }
-            if (tp.atc)
+            if (tp.atc && C > 1)
+                tc_store_pair(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + cc), cscale(J, filt[k]));
+            else if (tp.atc)
                 tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + cc), cscale(J, filt[k]));
             else
                 out0[o] = cscale(J, filt[k]);
@@ -757,7 +759,9 @@ __global__ void __launch_bounds__(LOGM > 0 ? 256 : 512, RAMAN ? 1 : (LOGM > 0 ? 
             const int ka = k & (M - 1), kb = (M - k) & (M - 1);
             const float2 X = real_spectrum(Ze[sw(ka) * C + cc], Ze[sw(kb) * C + cc], tws.get(k));
             const float wt = (k == 0 || k == M) ? inv : 2.f * inv;
-            if (tp.atc)  // the operand tiles of the Minv^T transform that follows
+            if (tp.atc && C > 1)  // the operand tiles of the Minv^T transform that follows
+                tc_store_pair(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + cc), cscale(X, wt));
+            else if (tp.atc)
                 tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + cc), cscale(X, wt));
             else
                 gE[(size_t)k * S + col0 + cc] = cscale(X, wt);

@@ -225,9 +225,7 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
     // ---- write J back: rows of NC columns ----
     __syncthreads();
     if (tp.atc)
-        tr_each_point<LOGM>(tid, S, col0, [&](int k, int c, size_t, int p) {
-            tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)(col0 + c), sm[p]);
-        });
+        tr_store_tiles<LOGM>(sm, tp.atc, tp.atc_nkt, tid, col0);
     else
         tr_each_point<LOGM>(tid, S, col0, [&](int, int, size_t o, int p) { Jout[o] = sm[p]; });
 }

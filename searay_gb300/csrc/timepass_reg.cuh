@@ -10,6 +10,7 @@
 
 #include "common.cuh"
 #include "dft_reg.cuh"
+#include "hankel_tc.cuh"
 
 template <int LOGM>
 struct TRegShape;
@@ -79,6 +80,23 @@ UPPE_DEV void tr_each_point(int tid, size_t S, size_t col0, Visit visit) {
 #pragma unroll 8
     for (int i = 0; i < G::M / KS; ++i, o += step) visit(k0 + KS * i, c, o, p + KS * i);
     if (k0 == 0) visit(G::M, c, o, p + G::M);
+}
+
+// The points of a block's columns into the operand tiles of the tensor-core Hankel transform (hankel_tc.cuh), eight
+// columns of a row to a thread: its 16-byte stores, eight neighbouring lanes' 128 contiguous bytes, against
+// four 2-byte stores a point.
+template <int LOGM>
+UPPE_DEV void tr_store_tiles(const float2* sm, uint8_t* atc, int nkt, int tid, size_t col0) {
+    using G = TReg<LOGM>;
+    const float* s = reinterpret_cast<const float*>(sm);
+#pragma unroll 1
+    for (int c8 = 0; c8 < G::NC; c8 += 8)
+        for (int i = tid; i < 2 * (G::M + 1); i += G::THREADS) {
+            float x[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) x[c] = s[2 * (c8 + c) * G::LD + i];  // re and im of w = i / 2 in turn
+            tc_store_row8(atc, nkt, i >> 1, i & 1, (int)col0 + c8, x);
+        }
 }
 
 // The radix-2 step of a 32-point DFT split over a lane pair (lanes t and t ^ 16 hold the two
