@@ -289,8 +289,7 @@ static cudaError_t launch_azimuth(UppeHandle* h, const float2* in, float2* out, 
 }
 
 cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* A, int which, float2* C0,
-                             float2* C1, const float2* qi, int NI, int NK, int spec_mode, float Cs, float Ce,
-                             StepArgs z);
+                             float2* C1, int NI, int NK, StepArgs z);
 
 size_t hankel_kmajor_len(int N1, int N2) {
     const size_t KP = (size_t)(N1 + GBK - 1) / GBK * GBK, LD = (size_t)(N1 + 3) / 4 * 4;
@@ -337,8 +336,7 @@ static cudaError_t run_simt(UppeHandle* h, GemmArgs& g) {
 template <int AMODE, int CMODE>
 static cudaError_t run_gemm(UppeHandle* h, GemmArgs& g) {
     if (h->cfg.precision == UPPE_PREC_MIXED)
-        return launch_hankel_tc(h, AMODE, CMODE, g.A, g.which, g.C0, g.C1, g.qi, g.NI, g.NK, g.spec_mode, g.Cs, g.Ce,
-                                g.z);
+        return launch_hankel_tc(h, AMODE, CMODE, g.A, g.which, g.C0, g.C1, g.NI, g.NK, g.z);
     return run_simt<AMODE, CMODE>(h, g);
 }
 
@@ -385,9 +383,11 @@ cudaError_t launch_real_cyl(UppeHandle* h, int mode, const float2* src, float2* 
     return launch_ikz(h, A, h->E);
 }
 
-// Forward transform of J (or of the incoming field for SPEC_LOAD) and the spectral update: fused
-// into the GEMM's epilogue in the SIMT form and on azimuthal grids (N2 > 1, the operand is the
-// azimuthal DFT in scratch); a separate elementwise pass after the tensor-core GEMM otherwise.
+// Forward transform of J (or of the incoming field for SPEC_LOAD) and the spectral update: fused into the GEMM's
+// epilogue in the SIMT form.  The tensor-core form stores its product over J (its pre-pass, or the azimuthal DFT, has
+// read J by then) and a separate elementwise pass applies S and the RK stage: the update reads five arrays a point,
+// which the GEMM's few blocks wait for and a pass over the whole grid streams (257 x 64 x 8 azimuthal: forward
+// transform with the update 24 us in the epilogue, 17 us apart; a ten-step pass 1.98 -> 1.82 ms).
 // z_next (stages whose estimate the next evaluation transforms at z_next): the tensor-core form's
 // spectral update also writes that inverse transform's operand tiles (k_spec_point).
 cudaError_t launch_spec_cyl(UppeHandle* h, int mode, const float2* src_real, float2* q_out, float2* qf_io,
@@ -403,21 +403,19 @@ cudaError_t launch_spec_cyl(UppeHandle* h, int mode, const float2* src_real, flo
         g.A = h->scratch;
     }
     g.C0 = q_out;
-    g.C1 = qf_io;
-    g.qi = qi;
-    g.Cs = Cs;
-    g.Ce = Ce;
-    g.spec_mode = mode;
     if (mode == SPEC_LOAD) return run_gemm<A_PLAIN, C_STORE>(h, g);
-    if (h->cfg.precision == UPPE_PREC_MIXED && g.A == h->J) {
-        // the tensor-core transform stores its product over J (its pre-pass has already read J into
-        // the operand tiles), then a separate pass applies S and the RK stage
+    if (h->cfg.precision == UPPE_PREC_MIXED) {
         g.C0 = h->J;
         cudaError_t err = run_gemm<A_PLAIN, C_STORE>(h, g);
         if (err != cudaSuccess) return err;
         return launch_spec_point(h, mode, h->J, q_out, qf_io, qi, Cs, Ce, z, h->N2 == 1 ? z_next : nullptr);
     }
-    return run_gemm<A_PLAIN, C_SPEC>(h, g);
+    g.C1 = qf_io;
+    g.qi = qi;
+    g.Cs = Cs;
+    g.Ce = Ce;
+    g.spec_mode = mode;
+    return run_simt<A_PLAIN, C_SPEC>(h, g);
 }
 
 // Adjoint transverse transforms on cylindrical grids (one azimuthal node) with the transposed folded

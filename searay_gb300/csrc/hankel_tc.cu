@@ -7,7 +7,7 @@
 //     A_hi B_hi + A_hi B_lo + A_lo B_hi in FP32 (the dropped A_lo B_lo is ~2^-18 of the product);
 //   * one elected thread issues tcgen05.mma (M=128, N=128, K=16) from shared-memory operands in the
 //     no-swizzle K-major core-matrix layout; the accumulator lives in tensor memory (TMEM) and is
-//     read back with tcgen05.ld for the fused epilogue (store, finish, or ODE RHS + RK stage);
+//     read back with tcgen05.ld for the fused epilogue (store, finish, or an adjoint's factor);
 //   * the A operand (the field with its propagator phase and i kz where the mode asks) is formed and
 //     split once per transform by k_hankel_tc_prep into tiles in that same layout, so every K step
 //     of an output tile is two contiguous 32 KB blocks (A and B), fetched by bulk copies into a ring
@@ -28,7 +28,7 @@
 // operand modes (TA_SADJ: the cotangent of S times conj(D2), the A operand of the adjoint ADJ_S)
 enum { TA_PLAIN = 0, TA_QPHASE_IKZ = 1, TA_QPHASE = 2, TA_PRESPLIT = 3, TA_SADJ = 4 };
 // epilogues (TC_QADJ / TC_FADJ: conj(D0) C and conj(exp(i(kz+kg)z)) C of the adjoint ADJ_E / ADJ_FIN)
-enum { TC_STORE = 0, TC_FINISH1 = 1, TC_SPEC = 2, TC_QADJ = 3, TC_FADJ = 4 };
+enum { TC_STORE = 0, TC_FINISH1 = 1, TC_QADJ = 3, TC_FADJ = 4 };  // values of hankel.cu's C_*
 
 struct TcArgs {
     const float2* A;
@@ -38,10 +38,7 @@ struct TcArgs {
     OpView op;
     float2* C0;
     float2* C1;
-    const float2* qi;
     int N0, N1, N2, NI, NK;
-    int spec_mode;
-    float Cs, Ce;
     StepArgs z;
     int* err;
 };
@@ -309,35 +306,10 @@ __global__ void __launch_bounds__(TcShape<TN>::THREADS, TcShape<TN>::MINB) k_han
             float2 r = cmul(cconj(propagator_factor(o, pa, 1.f)), v);
             if (CMODE == TC_QADJ) r = cmul(cconj(op_ikz(o)), r);
             g.C0[idx] = r;
-        } else if (CMODE == TC_FINISH1) {
+        } else {
             const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
             if (g.C0) g.C0[idx] = v;
             g.C1[idx] = op_field(g.op, o, v);
-        } else {
-            const float cond = (w < g.op.ncond) ? 0.f : 1.f;
-            const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
-            const float2 f = propagator_factor(o, pa, -1.f);
-            const float2 s = cscale(cmul_i(cmul(f, v)), 0.5f / o.kzr);
-            switch (g.spec_mode) {
-                case SPEC_STORE_K:
-                    g.C0[idx] = s;
-                    break;
-                case SPEC_STAGE1: {
-                    const float2 a = g.qi[idx];
-                    g.C1[idx] = cadd(a, cscale(s, g.Cs));
-                    g.C0[idx] = cscale(cadd(a, cscale(s, g.Ce)), cond);
-                } break;
-                case SPEC_STAGE23: {
-                    const float2 a = g.qi[idx];
-                    const float2 b = g.C1[idx];
-                    g.C1[idx] = cadd(b, cscale(s, g.Cs));
-                    g.C0[idx] = cscale(cadd(a, cscale(s, g.Ce)), cond);
-                } break;
-                default: {
-                    const float2 b = g.C1[idx];
-                    g.C0[idx] = cscale(cadd(b, cscale(s, g.Cs)), cond);
-                } break;
-            }
         }
     }
 }
@@ -374,8 +346,7 @@ static cudaError_t run_tc(UppeHandle* h, TcArgs& a) {
 // (its A_SADJ = 3 is TA_SADJ here); `which` selects the split matrix tiles: 0 Mfwd, 1 Minv,
 // 2 Mfwd^T, 3 Minv^T (the last two for the adjoint transforms).
 cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* A, int which, float2* C0,
-                             float2* C1, const float2* qi, int NI, int NK, int spec_mode, float Cs, float Ce,
-                             StepArgs z) {
+                             float2* C1, int NI, int NK, StepArgs z) {
     TcArgs a{};
     a.A = A;
     const uint8_t* const tiles[4] = {h->Mfwd_tc, h->Minv_tc, h->MfwdT_tc, h->MinvT_tc};
@@ -387,15 +358,11 @@ cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* 
     a.op = uppe_op_view(h);
     a.C0 = C0;
     a.C1 = C1;
-    a.qi = qi;
     a.N0 = h->N0;
     a.N1 = h->N1;
     a.N2 = h->N2;
     a.NI = NI;
     a.NK = NK;
-    a.spec_mode = spec_mode;
-    a.Cs = Cs;
-    a.Ce = Ce;
     a.z = z;
     a.err = h->dev_err;
     a.nwt = (h->N0 + TC_W - 1) / TC_W;
@@ -431,7 +398,6 @@ cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* 
         if (e != cudaSuccess) return e;
     }
     if (cmode == TC_STORE) return run_tc<TA_PRESPLIT, TC_STORE>(h, a);
-    if (cmode == TC_SPEC) return run_tc<TA_PRESPLIT, TC_SPEC>(h, a);
     if (cmode == TC_FINISH1) return run_tc<TA_PRESPLIT, TC_FINISH1>(h, a);
     if (cmode == TC_QADJ) return run_tc<TA_PRESPLIT, TC_QADJ>(h, a);
     if (cmode == TC_FADJ) return run_tc<TA_PRESPLIT, TC_FADJ>(h, a);
