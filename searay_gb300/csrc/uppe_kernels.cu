@@ -413,7 +413,7 @@ __global__ void k_spec_point(int mode, const float2* __restrict__ C, OpView opv,
         const float cond = (w < opv.ncond) ? 0.f : 1.f;
         const OpPoint o = op_at(opv, idx, opv.kg[w]);
         const float2 qw = spec_update(mode, idx, C[idx], o, cond, q_out, qf, qi, Cs, Ce, pa, true);
-        if (nx.Atc) {
+        if (nx.Atc && k < nx.nkt * TC_K) {  // (beyond: no tile of this row, where the modes end 64 nodes early)
             float2 a = make_float2(0.f, 0.f);
             if (k < nx.Nk) a = op_field(opv, o, cmul(propagator_factor(o, pn, 1.f), qw));
             tc_store_split(nx.Atc, nx.nwt, nx.nkt, 0, w, k, a);
