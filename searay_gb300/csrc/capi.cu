@@ -625,7 +625,7 @@ static int rk4_step_generic(UppeHandle* h, double z_phase, double L, double z_su
     }
     {
         // each stage estimate is transformed next at zn: the spectral update that forms it also forms
-        // that transform's operand (mixed form, one azimuthal node)
+        // that transform's operand (mixed form)
         StepArgs z = split_z(h, z_phase + 0.5 * dz);
         const StepArgs zn = split_z(h, z_phase + dz);
         CUDA_TRY(h, eval_to_J(h, h->q, z));

@@ -9,6 +9,7 @@
 // The azimuthal FFT (FFT_axis2/IFFT_axis2, fft.cl:401-441) of grids with N2 > 1 runs as a separate
 // DFT pass around the GEMM.
 #include "common.cuh"
+#include "hankel_tc.cuh"
 #include "time_common.cuh"
 #include "uppe_internal.h"
 
@@ -276,6 +277,25 @@ __global__ void k_azimuth_dft(const float2* __restrict__ in, float2* __restrict_
     }
 }
 
+// The forward azimuthal DFT of the mixed form, its outputs split straight into the operand tiles of the tensor-core
+// transform that follows (tile order of k_hankel_tc_prep).  Eight neighbouring lanes take eight radial nodes
+// of one azimuthal mode: their 2-byte stores fill 16-byte rows, their loads of one azimuthal node share sectors
+// with those of the warp's other modes.
+__global__ void k_azimuth_tiles(const float2* __restrict__ in, uint8_t* __restrict__ Atc, int N0, int N1, int N2,
+                                int logN2, int nwt, int nkt, const float2* __restrict__ tw, int twLog) {
+    const size_t rows = (size_t)N0 * N1, n = ((rows + 7) >> 3) << (3 + logN2);
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const int j = (int)(i >> 3) & (N2 - 1);
+        const size_t row = ((i >> (3 + logN2)) << 3) + (i & 7);
+        if (row >= rows) continue;
+        const float2* src = in + row * N2;
+        float2 acc = make_float2(0.f, 0.f);
+        for (int mm = 0; mm < N2; ++mm)
+            acc = cadd(acc, cmul(src[mm], __ldg(&tw[((j * mm) & (N2 - 1)) << (twLog - logN2)])));
+        tc_store_split(Atc, nwt, nkt, j, (int)(row / N1), (int)(row % N1), acc);
+    }
+}
+
 static cudaError_t launch_azimuth(UppeHandle* h, const float2* in, float2* out, bool inv) {
     const int logN2 = ilog2_exact(h->N2);
     const size_t rows = (size_t)h->N0 * h->N1;
@@ -290,6 +310,18 @@ static cudaError_t launch_azimuth(UppeHandle* h, const float2* in, float2* out, 
 
 cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* A, int which, float2* C0,
                              float2* C1, int NI, int NK, StepArgs z);
+
+static cudaError_t launch_azimuth_tiles(UppeHandle* h, const float2* in) {
+    const int logN2 = ilog2_exact(h->N2);
+    const size_t n = ((((size_t)h->N0 * h->N1 + 7) >> 3) << 3) * h->N2;
+    unsigned blocks = (unsigned)((n + 255) / 256);
+    if (blocks > 152 * 16) blocks = 152 * 16;
+    h->launches++;
+    h->atc_next = 0;
+    k_azimuth_tiles<<<blocks, 256, 0, h->stream>>>(in, h->Atc, h->N0, h->N1, h->N2, logN2, (h->N0 + TC_W - 1) / TC_W,
+                                                   (h->N1 + TC_K - 1) / TC_K, h->tw, h->twLog);
+    return cudaGetLastError();
+}
 
 size_t hankel_kmajor_len(int N1, int N2) {
     const size_t KP = (size_t)(N1 + GBK - 1) / GBK * GBK, LD = (size_t)(N1 + 3) / 4 * 4;
@@ -398,9 +430,17 @@ cudaError_t launch_spec_cyl(UppeHandle* h, int mode, const float2* src_real, flo
     g.NK = h->N1;
     g.A = src_real;
     if (h->N2 > 1) {
-        cudaError_t err = launch_azimuth(h, src_real, h->scratch, false);
-        if (err != cudaSuccess) return err;
         g.A = h->scratch;
+        // (a ragged last tile needs the zeros that the transform's own pre-pass writes, unless it is the only one)
+        const bool tiles = h->cfg.precision == UPPE_PREC_MIXED && h->tc_next && h->Atc &&
+                           (h->N1 % TC_K == 0 || h->N1 < TC_K);
+        cudaError_t err = tiles ? launch_azimuth_tiles(h, src_real) : launch_azimuth(h, src_real, h->scratch, false);
+        if (err != cudaSuccess) return err;
+        if (tiles) {
+            h->atc_fwd = 1;
+            h->atc_fwd_which = 0;
+            h->atc_fwd_src = h->scratch;
+        }
     }
     g.C0 = q_out;
     if (mode == SPEC_LOAD) return run_gemm<A_PLAIN, C_STORE>(h, g);
@@ -408,7 +448,7 @@ cudaError_t launch_spec_cyl(UppeHandle* h, int mode, const float2* src_real, flo
         g.C0 = h->J;
         cudaError_t err = run_gemm<A_PLAIN, C_STORE>(h, g);
         if (err != cudaSuccess) return err;
-        return launch_spec_point(h, mode, h->J, q_out, qf_io, qi, Cs, Ce, z, h->N2 == 1 ? z_next : nullptr);
+        return launch_spec_point(h, mode, h->J, q_out, qf_io, qi, Cs, Ce, z, z_next);
     }
     g.C1 = qf_io;
     g.qi = qi;

@@ -404,11 +404,12 @@ cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* 
     return cudaErrorInvalidValue;
 }
 
-// The operand of the next inverse transform, for the spectral update that writes it (N2 = 1): the
+// The operand of the next inverse transform, for the spectral update that writes it: the
 // tile counts of the Minv transform and its z.
 TcNext hankel_tc_next(const UppeHandle* h, StepArgs z_next) {
     TcNext nx;
     nx.Atc = h->Atc;
+    nx.logN2 = ilog2_exact(h->N2);
     nx.nwt = (h->N0 + TC_W - 1) / TC_W;
     nx.nkt = (h->Nk + TC_K - 1) / TC_K;
     nx.Nk = h->Nk;

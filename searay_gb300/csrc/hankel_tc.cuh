@@ -89,6 +89,7 @@ __device__ __forceinline__ void tc_store_row8(uint8_t* __restrict__ Atc, int nkt
 // Atc NULL when not asked.
 struct TcNext {
     uint8_t* Atc;
+    int logN2;         // azimuthal nodes (the fast axis of the field)
     int nwt, nkt, Nk;  // tile counts of the inverse transform (reduction over the Nk radial modes)
     StepArgs z;        // the next evaluation's z
 };

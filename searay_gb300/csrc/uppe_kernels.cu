@@ -394,7 +394,7 @@ __global__ void k_adj_rk(int mode, const float2* __restrict__ lam_out, float2* _
 // The spectral update of every point from the transformed current C (the ODE right-hand side and the
 // RK stage of spec_update), as a separate pass after a tensor-core transform that stored C: many
 // warps per multiprocessor hide the latency of its operand reads, which the GEMM's own epilogue,
-// with one block per multiprocessor, does not.  With nx.Atc set (one azimuthal node) it also writes
+// with one block per multiprocessor, does not.  With nx.Atc set it also writes
 // the operand of the next inverse transform, i kz exp(i (kz + kg) z_next) qw of the new stage
 // estimate qw, split into the transform's bf16 tiles (zero beyond the Nk radial modes), which
 // k_hankel_tc_prep would otherwise form from qw.
@@ -413,10 +413,11 @@ __global__ void k_spec_point(int mode, const float2* __restrict__ C, OpView opv,
         const float cond = (w < opv.ncond) ? 0.f : 1.f;
         const OpPoint o = op_at(opv, idx, opv.kg[w]);
         const float2 qw = spec_update(mode, idx, C[idx], o, cond, q_out, qf, qi, Cs, Ce, pa, true);
-        if (nx.Atc && k < nx.nkt * TC_K) {  // (beyond: no tile of this row, where the modes end 64 nodes early)
+        const int kr = k >> nx.logN2;
+        if (nx.Atc && kr < nx.nkt * TC_K) {  // (beyond: no tile of this row, where the modes end 64 nodes early)
             float2 a = make_float2(0.f, 0.f);
-            if (k < nx.Nk) a = op_field(opv, o, cmul(propagator_factor(o, pn, 1.f), qw));
-            tc_store_split(nx.Atc, nx.nwt, nx.nkt, 0, w, k, a);
+            if (kr < nx.Nk) a = op_field(opv, o, cmul(propagator_factor(o, pn, 1.f), qw));
+            tc_store_split(nx.Atc, nx.nwt, nx.nkt, k & ((1 << nx.logN2) - 1), w, kr, a);
         }
         w += dw;
         k += dk;
