@@ -19,6 +19,7 @@
 
 #include "common.cuh"
 #include "fft_smem.cuh"
+#include "hankel_tc.cuh"
 #include "time_common.cuh"
 #include "uppe_internal.h"
 
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
     const size_t col0 = (size_t)blockIdx.x * C;
     const bool ionize = tp.rate_form != UPPE_RATE_NONE;
     const TwHalfShared tws{twl, logN0};
+    pdl_begin();
 
     // ---- 1. stage A[k][c] (asynchronous copies), then i w A and the two inverse FFTs ----
     if (C >= 2) {
@@ -182,7 +184,12 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
         if (mode == TIME_J) {
             float2 J = cmul_mi(cscale(ZE[it], __ldg(&wv[k])));
             if (ionize) J = cadd(J, ZA[it]);
-            out0[o] = J;
+            if (tp.atc && C > 1)  // the forward tensor-core transform's operand tiles
+                tc_store_pair(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)col0 + (it & (C - 1)), J);
+            else if (tp.atc)
+                tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)col0, J);
+            else
+                out0[o] = J;
         } else {
             if (out0) out0[o] = ZE[it];
             if (out1) out1[o] = ionize ? ZA[it] : make_float2(0.f, 0.f);
@@ -218,8 +225,8 @@ cudaError_t launch_time_env(UppeHandle* h, int mode, const float2* A, float2* ou
     const int form = h->rot_pairs > 0 ? (h->rot_conv ? 2 : 1) : 0;
     h->launches++;
 #define UPPE_ENV_LAUNCH(F_, SPT_)                                                                                      \
-    k_time_env<F_, SPT_><<<h->S / h->time_cols, R / SPT_, smem, h->stream>>>(mode, A, out0, out1, h->ng, h->w, h->tw, \
-                                                                            h->twLog, tp)
+    launch_pdl(k_time_env<F_, SPT_>, dim3(h->S / h->time_cols), dim3(R / SPT_), smem, h->stream, mode, A, out0, out1, \
+               h->ng, h->w, h->tw, h->twLog, tp)
     if (form == 0) UPPE_ENV_LAUNCH(0, 16);
     else if (form == 1) UPPE_ENV_LAUNCH(1, 16);
     else if (R / 8 <= 512 && R >= 32) UPPE_ENV_LAUNCH(2, 8);
