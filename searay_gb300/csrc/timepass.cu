@@ -43,8 +43,8 @@ __device__ __forceinline__ float2 real_spectrum(float2 Za, float2 Zb_raw, float2
 // array of Nt C over Zj and Zr, Zr following Zj; 3: one block per multiprocessor, 4: two.
 template <int ET, int LOGM = 0, int LOGC = -1, int RAMAN = 0>
 // (three blocks per multiprocessor where shared memory allows it: M <= 512)
-__global__ void __launch_bounds__(ET == 16 ? 256 : 512,
-                                  RAMAN ? 2 - (RAMAN & 1) : (ET == 16 ? 3 : ((LOGM > 0 && LOGM <= 9) ? 3 : 2))) k_time(int mode, const float2* __restrict__ E, float2* __restrict__ out0,
+__global__ void __launch_bounds__(ET == 16 || (LOGM > 0 && LOGM <= 7) ? 256 : 512,
+                                  RAMAN ? 2 - (RAMAN & 1) : (ET == 16 || (LOGM > 0 && LOGM <= 9) ? 3 : 2)) k_time(int mode, const float2* __restrict__ E, float2* __restrict__ out0,
                                                   float2* __restrict__ out1, const float* __restrict__ ng,
                                                   const float* __restrict__ wv, const float* __restrict__ filt,
                                                   const float2* __restrict__ tw, int twLog, TimeParams tp) {
@@ -314,8 +314,10 @@ __global__ void __launch_bounds__(ET == 16 ? 256 : 512,
 }
 
 // The time-pass shapes with compile-time sizes: C Nt = 8192 with 16 samples per thread (512 threads),
-// M = 256 .. 2048.
-#define UPPE_TIME_CT(X) X(8, 4) X(9, 3) X(10, 2) X(11, 1)
+// M = 256 .. 2048; and the 16 columns per block of shorter time axes, M = 64 and 128, which with sizes from the
+// parameters waited for their index arithmetic and for one sample's rate at a time (time pass, us: 129 x 64 x 32
+// 22.8 -> 17.7, 129 x 128 x 128 40.8 -> 30.3, 65 x 128 x 128 24.9 -> 20.8).
+#define UPPE_TIME_CT(X) X(6, 4) X(7, 4) X(8, 4) X(9, 3) X(10, 2) X(11, 1)
 
 cudaError_t uppe_configure_time_kernel(size_t smem_bytes) {
     cudaError_t e = cudaFuncSetAttribute(k_time<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
