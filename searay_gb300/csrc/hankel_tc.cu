@@ -76,17 +76,17 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase, int* er
     return false;
 }
 
-// Output-tile shapes of the GEMM: TN = 128 columns per tile, 512 threads, three 64 KB stages, one
-// block per multiprocessor (the shape in use); TN = 64, 256 threads, two 48 KB stages, two blocks
-// per multiprocessor, gave the same results bit for bit but ran slower (18.7 against 15.7 us per
-// inverse transform at 2049 x 512: every A tile is fetched by twice as many blocks).  A stage is
+// Output-tile shapes of the GEMM, one block of 512 threads per multiprocessor: TN = 128 columns per tile and three
+// 64 KB stages; TN = 64 and four 48 KB stages where twice the blocks of the wide tile still fit the chip at once,
+// which shortens a block's copies, products and epilogue: transform with its update, us, wide | narrow: 2049 x 256
+// (66 | 132 blocks) 8.0 | 7.1, 1025 x 256 8.3 | 6.6; 2049 x 512 (132 blocks wide) is slower narrow, every A tile
+// being fetched by twice as many blocks (15.7 | 18.7).  The same bits in both.  A stage is
 // [A_hi | A_lo | B_hi | B_lo]; a B tile of TN rows is the upper or lower half (contiguous 8 KB) of the
 // 128-row split matrix tiles.
 template <int TN>
 struct TcShape {
-    static constexpr int THREADS = TN == 128 ? 512 : 256;
-    static constexpr int NSTAGE = TN == 128 ? 3 : 2;
-    static constexpr int MINB = TN == 128 ? 1 : 2;
+    static constexpr int THREADS = 512;
+    static constexpr int NSTAGE = TN == 128 ? 3 : 4;
     static constexpr uint32_t BTILE = (uint32_t)TN * TC_K * 2;  // bytes of one B operand (hi or lo)
     static constexpr uint32_t STAGE = 2 * TC_TILE_BYTES + 2 * BTILE;
     static constexpr int LD = TN + 1;  // padded row of the epilogue staging tile (float2)
@@ -166,7 +166,7 @@ __global__ void __launch_bounds__(256) k_hankel_tc_prep(TcArgs g, uint8_t* __res
 // step (committed to the stage's `done` mbarrier), and refills the stage of the previous step once
 // its MMAs have completed, so the copies run NSTAGE - 1 steps ahead of the tensor core.
 template <int AMODE, int CMODE, int TN>
-__global__ void __launch_bounds__(TcShape<TN>::THREADS, TcShape<TN>::MINB) k_hankel_tc(TcArgs g) {
+__global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g) {
     using SH = TcShape<TN>;
     constexpr int NST = SH::NSTAGE, TT = SH::THREADS, LD = SH::LD;
     pdl_launch_next();
@@ -348,7 +348,8 @@ static cudaError_t run_tc_shape(UppeHandle* h, TcArgs& a) {
 
 template <int AMODE, int CMODE>
 static cudaError_t run_tc(UppeHandle* h, TcArgs& a) {
-    return run_tc_shape<AMODE, CMODE, 128>(h, a);
+    const long blocks = (long)((a.NI + 127) / 128) * ((a.N0 + TC_W - 1) / TC_W) * a.N2;
+    return 2 * blocks <= h->num_sms ? run_tc_shape<AMODE, CMODE, 64>(h, a) : run_tc_shape<AMODE, CMODE, 128>(h, a);
 }
 
 // Entry used by hankel.cu in the mixed-precision form.  amode/cmode follow hankel.cu's A_*/C_* codes

@@ -812,7 +812,7 @@ __global__ void __launch_bounds__(LOGM > 0 ? 256 : 512, RAMAN ? 1 : (LOGM > 0 ? 
 }
 
 // The adjoint time-pass shapes with compile-time sizes: 2048 complex elements per block (256 threads).
-#define UPPE_TIME_ADJ_CT(X) X(8, 3) X(9, 2) X(10, 1) X(11, 0)
+#define UPPE_TIME_ADJ_CT(X) X(6, 4) X(7, 4) X(8, 3) X(9, 2) X(10, 1) X(11, 0)
 
 cudaError_t uppe_configure_time_adj_kernel(size_t smem_bytes) {
     cudaError_t e = cudaFuncSetAttribute(k_time_adj<>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
