@@ -7,7 +7,8 @@
 //     A_hi B_hi + A_hi B_lo + A_lo B_hi in FP32 (the dropped A_lo B_lo is ~2^-18 of the product);
 //   * one elected thread issues tcgen05.mma (M=128, N=128, K=16) from shared-memory operands in the
 //     no-swizzle K-major core-matrix layout; the accumulator lives in tensor memory (TMEM) and is
-//     read back with tcgen05.ld for the fused epilogue (store, finish, or an adjoint's factor);
+//     read back with tcgen05.ld and stored; the finish's i kz and the adjoint's factors are a
+//     pass of their own over the product (k_hankel_tc_point);
 //   * the A operand (the field with its propagator phase and i kz where the mode asks) is formed and
 //     split once per transform by k_hankel_tc_prep into tiles in that same layout, so every K step
 //     of an output tile is two contiguous 32 KB blocks (A and B), fetched by bulk copies into a ring
@@ -26,18 +27,18 @@
 #define TC_WAIT_LIMIT (1 << 24)
 
 // operand modes (TA_SADJ: the cotangent of S times conj(D2), the A operand of the adjoint ADJ_S)
-enum { TA_PLAIN = 0, TA_QPHASE_IKZ = 1, TA_QPHASE = 2, TA_PRESPLIT = 3, TA_SADJ = 4 };
-// epilogues (TC_QADJ / TC_FADJ: conj(D0) C and conj(exp(i(kz+kg)z)) C of the adjoint ADJ_E / ADJ_FIN)
-enum { TC_STORE = 0, TC_FINISH1 = 1, TC_QADJ = 3, TC_FADJ = 4 };  // values of hankel.cu's C_*
+enum { TA_PLAIN = 0, TA_QPHASE_IKZ = 1, TA_QPHASE = 2, TA_SADJ = 4 };
+// results (hankel.cu's C_*): the product C; A = C and E = i kz C (FINISH1); conj(D0) C (QADJ) and
+// conj(exp(i(kz+kg)z)) C (FADJ) of the adjoint ADJ_E / ADJ_FIN
+enum { TC_STORE = 0, TC_FINISH1 = 1, TC_QADJ = 3, TC_FADJ = 4 };
 
 struct TcArgs {
     const float2* A;
     const uint8_t* Btc;  // split matrix tiles [N2][nit][nkt][hi 16 KB | lo 16 KB]
-    const uint8_t* Atc;  // split field tiles [N2][nwt][nkt][hi 16 KB | lo 16 KB] (TA_PRESPLIT)
+    const uint8_t* Atc;  // split field tiles [N2][nwt][nkt][hi 16 KB | lo 16 KB]
     int nit, nkt, nwt;
     OpView op;
-    float2* C0;
-    float2* C1;
+    float2* C;
     int N0, N1, N2, NI, NK;
     StepArgs z;
     int* err;
@@ -160,17 +161,15 @@ __global__ void __launch_bounds__(256) k_hankel_tc_prep(TcArgs g, uint8_t* __res
     tc_store_split(Atc, g.nwt, g.nkt, m, w, k, v);
 }
 
-// The GEMM of one output tile (64 frequencies x TN columns) on pre-split operand tiles (AMODE =
-// TA_PRESPLIT).  Thread 0 drives a ring of NSTAGE stages: it issues the A and B tiles of a K step
+// The GEMM of one output tile (64 frequencies x TN columns) on pre-split operand tiles.  Thread 0 drives a ring of NSTAGE stages: it issues the A and B tiles of a K step
 // as bulk copies that complete on the stage's `full` mbarrier, waits for them, issues the MMAs of the
 // step (committed to the stage's `done` mbarrier), and refills the stage of the previous step once
 // its MMAs have completed, so the copies run NSTAGE - 1 steps ahead of the tensor core.
-template <int AMODE, int CMODE, int TN>
+template <int TN>
 __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g) {
     using SH = TcShape<TN>;
     constexpr int NST = SH::NSTAGE, TT = SH::THREADS, LD = SH::LD;
     pdl_launch_next();
-    static_assert(AMODE == TA_PRESPLIT, "the GEMM reads pre-split operand tiles");
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // NST pipeline stages of [A_hi | A_lo | B_hi | B_lo] (1024-byte aligned), reused afterwards
     // as the epilogue staging tile
@@ -185,7 +184,6 @@ __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g)
     const int w0 = blockIdx.y * TC_W;
     const int it = blockIdx.x;
     const int i0 = it * TN;
-    const PhaseArgs pa{g.z.zhi, g.z.zlo, g.z.plain};
     const uint32_t tiles_a = smem_u32(tiles);
     const uint32_t full0 = smem_u32(&full[0]), done0 = smem_u32(&done[0]);  // stage s at + 8 s
 
@@ -301,26 +299,43 @@ __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g)
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem_d), "r"(TN));
     if (aborted) return;
 
-    // ---- fused epilogue, coalesced along the output columns ----
+    // ---- store, coalesced along the output columns ----
     for (int e = tid; e < TC_W * TN; e += TT) {
         const int col = e & (TN - 1), wle = e / TN;
         const int w = w0 + wle, i = i0 + col;
-        if (w >= g.N0 || i >= g.NI) continue;
-        const float2 v = stage[wle * LD + col];
-        const size_t idx = ((size_t)w * g.N1 + i) * g.N2 + m;
-        if (CMODE == TC_STORE) {
-            g.C0[idx] = v;
-        } else if (CMODE == TC_QADJ || CMODE == TC_FADJ) {
-            const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
-            float2 r = cmul(cconj(propagator_factor(o, pa, 1.f)), v);
-            if (CMODE == TC_QADJ) r = cmul(cconj(op_ikz(o)), r);
-            g.C0[idx] = r;
+        if (w < g.N0 && i < g.NI) g.C[((size_t)w * g.N1 + i) * g.N2 + m] = stage[wle * LD + col];
+    }
+}
+
+// The pointwise factor on a stored product (in may be out).  As the GEMM's epilogue it ran on the few multiprocessors
+// that have a tile, each point's operands waiting for the stores of the point before: 1025 x 256 (34 blocks), transform
+// with conj(D0) 17.2 us against 8.3 without; apart, a gradient of four steps takes 2.05 ms instead of 2.09.
+template <int CMODE>
+__global__ void __launch_bounds__(256) k_hankel_tc_point(const float2* in, float2* out, OpView op, size_t n, int S,
+                                                        StepArgs z) {
+    pdl_begin();
+    const PhaseArgs pa{z.zhi, z.zlo, z.plain};
+    for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
+        const OpPoint o = op_at(op, idx, op.kg[idx / (size_t)S]);
+        const float2 v = in[idx];
+        if constexpr (CMODE == TC_FINISH1) {
+            out[idx] = op_field(op, o, v);
         } else {
-            const OpPoint o = op_at(g.op, idx, g.op.kg[w]);
-            if (g.C0) g.C0[idx] = v;
-            g.C1[idx] = op_field(g.op, o, v);
+            float2 r = cmul(cconj(propagator_factor(o, pa, 1.f)), v);
+            if constexpr (CMODE == TC_QADJ) r = cmul(cconj(op_ikz(o)), r);
+            out[idx] = r;
         }
     }
+}
+
+template <int CMODE>
+static cudaError_t run_point(UppeHandle* h, const float2* in, float2* out, StepArgs z) {
+    size_t blocks = (h->P + 255) / 256;
+    if (blocks > 152 * 8) blocks = 152 * 8;
+    h->launches++;
+    launch_pdl(k_hankel_tc_point<CMODE>, dim3((unsigned)blocks), dim3(256), 0, h->stream, in, out, uppe_op_view(h), h->P,
+               h->S, z);
+    return cudaGetLastError();
 }
 
 template <int TN>
@@ -330,26 +345,25 @@ static size_t tc_smem_bytes() {
     return (ops > stage ? ops : stage) + 1024;  // + alignment slack
 }
 
-template <int AMODE, int CMODE, int TN>
+template <int TN>
 static cudaError_t run_tc_shape(UppeHandle* h, TcArgs& a) {
     static bool configured = false;
     const size_t smem = tc_smem_bytes<TN>();
     if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(k_hankel_tc<AMODE, CMODE, TN>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e =
+            cudaFuncSetAttribute(k_hankel_tc<TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         configured = true;
     }
     dim3 grid((a.NI + TN - 1) / TN, (a.N0 + TC_W - 1) / TC_W, a.N2);
     h->launches++;
-    launch_pdl(k_hankel_tc<AMODE, CMODE, TN>, grid, dim3(TcShape<TN>::THREADS), smem, h->stream, a);
+    launch_pdl(k_hankel_tc<TN>, grid, dim3(TcShape<TN>::THREADS), smem, h->stream, a);
     return cudaGetLastError();
 }
 
-template <int AMODE, int CMODE>
 static cudaError_t run_tc(UppeHandle* h, TcArgs& a) {
     const long blocks = (long)((a.NI + 127) / 128) * ((a.N0 + TC_W - 1) / TC_W) * a.N2;
-    return 2 * blocks <= h->num_sms ? run_tc_shape<AMODE, CMODE, 64>(h, a) : run_tc_shape<AMODE, CMODE, 128>(h, a);
+    return 2 * blocks <= h->num_sms ? run_tc_shape<64>(h, a) : run_tc_shape<128>(h, a);
 }
 
 // Entry used by hankel.cu in the mixed-precision form.  amode/cmode follow hankel.cu's A_*/C_* codes
@@ -366,8 +380,7 @@ cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* 
     a.nit = (NI + TC_N - 1) / TC_N;
     a.nkt = (NK + TC_K - 1) / TC_K;
     a.op = uppe_op_view(h);
-    a.C0 = C0;
-    a.C1 = C1;
+    a.C = C0 ? C0 : C1;
     a.N0 = h->N0;
     a.N1 = h->N1;
     a.N2 = h->N2;
@@ -407,10 +420,11 @@ cudaError_t launch_hankel_tc(UppeHandle* h, int amode, int cmode, const float2* 
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    if (cmode == TC_STORE) return run_tc<TA_PRESPLIT, TC_STORE>(h, a);
-    if (cmode == TC_FINISH1) return run_tc<TA_PRESPLIT, TC_FINISH1>(h, a);
-    if (cmode == TC_QADJ) return run_tc<TA_PRESPLIT, TC_QADJ>(h, a);
-    if (cmode == TC_FADJ) return run_tc<TA_PRESPLIT, TC_FADJ>(h, a);
+    cudaError_t e = run_tc(h, a);
+    if (e != cudaSuccess || cmode == TC_STORE) return e;
+    if (cmode == TC_FINISH1) return run_point<TC_FINISH1>(h, a.C, C1, z);
+    if (cmode == TC_QADJ) return run_point<TC_QADJ>(h, a.C, C0, z);
+    if (cmode == TC_FADJ) return run_point<TC_FADJ>(h, a.C, C0, z);
     return cudaErrorInvalidValue;
 }
 
