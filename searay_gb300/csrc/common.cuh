@@ -13,11 +13,9 @@
 // grid's blocks are then resident, so the next grid's waiting blocks can never keep one of them
 // out), then waits for the previous kernel to complete with its memory visible
 // (griddepcontrol.wait; it returns at once when there is none, or the kernel was launched plainly).
-UPPE_DEV void pdl_launch_next() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-UPPE_DEV void pdl_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 UPPE_DEV void pdl_begin() {
-    pdl_launch_next();
-    pdl_wait();
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
 }
 
 #ifdef __CUDACC__

@@ -169,7 +169,7 @@ template <int TN>
 __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g) {
     using SH = TcShape<TN>;
     constexpr int NST = SH::NSTAGE, TT = SH::THREADS, LD = SH::LD;
-    pdl_launch_next();
+    pdl_begin();
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     // NST pipeline stages of [A_hi | A_lo | B_hi | B_lo] (1024-byte aligned), reused afterwards
     // as the epilogue staging tile
@@ -213,14 +213,11 @@ __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g)
     const uint8_t* Abase = g.Atc + ((size_t)m * g.nwt + w0 / TC_W) * nkt * (size_t)(2 * TC_TILE_BYTES);
 
     if (tid == 0) {
-        const auto load_a = [&](int kt, int s2) {
-            bulk_g2s(tiles_a + (uint32_t)s2 * SH::STAGE, Abase + (size_t)kt * (2 * TC_TILE_BYTES), 2 * TC_TILE_BYTES,
-                     full0 + 8u * s2);
-        };
-        const auto load_b = [&](int kt, int s2) {
+        const auto load = [&](int kt, int s2) {
             const uint32_t st = tiles_a + (uint32_t)s2 * SH::STAGE, fb = full0 + 8u * s2;
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(fb), "r"(SH::STAGE)
                          : "memory");
+            bulk_g2s(st, Abase + (size_t)kt * (2 * TC_TILE_BYTES), 2 * TC_TILE_BYTES, fb);
             const uint8_t* bk = Bbase + (size_t)kt * (2 * TC_TILE_BYTES);
             if constexpr (TN == 128) {
                 bulk_g2s(st + 2 * TC_TILE_BYTES, bk, 2 * TC_TILE_BYTES, fb);
@@ -233,10 +230,7 @@ __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g)
         int landed = 0;  // K steps whose copies have been waited for
         int mmas = 0;    // K steps whose MMAs are issued
         bool ok = true;
-        // the matrix does not depend on the kernel before this one: its first tiles are on their way before the wait
-        for (int s2 = 0; s2 < nkt && s2 < NST; ++s2) load_b(s2, s2);
-        pdl_wait();
-        for (; issued < nkt && issued < NST; ++issued) load_a(issued, issued);
+        for (; issued < nkt && issued < NST; ++issued) load(issued, issued);
         for (int kt = 0; kt < nkt && ok; ++kt) {
             const int s2 = kt % NST;
             ok = mbar_wait(full0 + 8u * s2, (uint32_t)((kt / NST) & 1), g.err);
@@ -248,8 +242,7 @@ __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g)
                 const int sp = (kt - 1) % NST;  // == issued % NST
                 ok = mbar_wait(done0 + 8u * sp, (uint32_t)(((kt - 1) / NST) & 1), g.err);
                 if (!ok) break;
-                load_b(issued, sp);
-                load_a(issued, sp);
+                load(issued, sp);
                 ++issued;
             }
         }
@@ -263,8 +256,6 @@ __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g)
                 mbar_wait(done0 + 8u * ((mmas - 1) % NST), (uint32_t)(((mmas - 1) / NST) & 1), nullptr);
             aborted = 1;
         }
-    } else {
-        pdl_wait();  // (the epilogue writes what the kernel before this one may read)
     }
     asm volatile("tcgen05.fence::after_thread_sync;\n");
     __syncthreads();
