@@ -337,6 +337,43 @@ cudaError_t uppe_configure_time_kernel(size_t smem_bytes) {
     return e;
 }
 
+// The field below which the rate is not representable in FP32, of the configured rate model: once per handle (some 150
+// logarithms of host time, which every launch of a time pass used to take).
+float uppe_em_min(const UppeConfig& c) {
+    const double log2e = 1.4426950408889634;
+    float em_min = 0.f;
+    if (c.rate_form != UPPE_RATE_NONE) {
+        // log2(rate) as a function of Em (atomic units); it rises from -inf at Em -> 0 for physical
+        // rate models.  Bisect for the Em where it crosses -150, well below FP32's 2^-126.
+        auto log2rate = [&](double em) {
+            if (c.rate_form == UPPE_RATE_EXPLICIT)
+                return log2(c.rate_conv * c.c_pre) + c.c_pow * log2(em) + c.c_exp * log2e / em;
+            const double L = log(em);
+            double p = c.clog[5];
+            for (int i = 4; i >= 0; --i) p = p * L + c.clog[i];
+            return log2(c.rate_conv) + p * log2e;
+        };
+        double lo = c.field_cutoff, hi = 10.0;
+        if (log2rate(lo) < -150.0 && log2rate(hi) > -150.0) {
+            for (int it = 0; it < 80; ++it) {
+                const double mid = 0.5 * (lo + hi);
+                if (log2rate(mid) < -150.0)
+                    lo = mid;
+                else
+                    hi = mid;
+            }
+            // only trust the threshold if the rate really stays below it on [cutoff, lo]
+            bool mono = true;
+            for (int i = 0; i <= 64; ++i) {
+                const double em = c.field_cutoff + (lo - c.field_cutoff) * i / 64.0;
+                if (log2rate(em) > -150.0) mono = false;
+            }
+            if (mono) em_min = (float)lo;
+        }
+    }
+    return em_min;
+}
+
 TimeParams uppe_time_params(const UppeHandle* h) {
     const UppeConfig& c = h->cfg;
     TimeParams tp;
@@ -378,36 +415,7 @@ TimeParams uppe_time_params(const UppeHandle* h) {
         tp.atc_nwt = (h->N0 + TC_W - 1) / TC_W;
         tp.atc_nkt = (h->N1 + TC_K - 1) / TC_K;
     }
-    tp.em_min = 0.f;
-    if (c.rate_form != UPPE_RATE_NONE) {
-        // log2(rate) as a function of Em (atomic units); it rises from -inf at Em -> 0 for physical
-        // rate models.  Bisect for the Em where it crosses -150, well below FP32's 2^-126.
-        auto log2rate = [&](double em) {
-            if (c.rate_form == UPPE_RATE_EXPLICIT)
-                return log2(c.rate_conv * c.c_pre) + c.c_pow * log2(em) + c.c_exp * log2e / em;
-            const double L = log(em);
-            double p = c.clog[5];
-            for (int i = 4; i >= 0; --i) p = p * L + c.clog[i];
-            return log2(c.rate_conv) + p * log2e;
-        };
-        double lo = c.field_cutoff, hi = 10.0;
-        if (log2rate(lo) < -150.0 && log2rate(hi) > -150.0) {
-            for (int it = 0; it < 80; ++it) {
-                const double mid = 0.5 * (lo + hi);
-                if (log2rate(mid) < -150.0)
-                    lo = mid;
-                else
-                    hi = mid;
-            }
-            // only trust the threshold if the rate really stays below it on [cutoff, lo]
-            bool mono = true;
-            for (int i = 0; i <= 64; ++i) {
-                const double em = c.field_cutoff + (lo - c.field_cutoff) * i / 64.0;
-                if (log2rate(em) > -150.0) mono = false;
-            }
-            if (mono) tp.em_min = (float)lo;
-        }
-    }
+    tp.em_min = h->em_min;
     return tp;
 }
 

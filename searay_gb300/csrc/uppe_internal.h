@@ -101,6 +101,7 @@ struct UppeHandle {
     double max_abs_K;   // max |Re kz + kg| of the current operator
     double max_Ki;      // max Im kz of the current operator
     double redchi3;        // chi3 / density reference in use (uppe_set_chi3)
+    float em_min;          // field below which the ionization rate counts as zero (uppe_em_min)
     int rot_pairs;         // rotational Raman transitions in use (uppe_set_rotator), in pairs; 0 = none
     float* rot;            // their tables: [rot_pairs][80] then the phasors [rot_pairs][Nt/16] (float4)
     int rot_conv;          // the convolution's tables follow (3 Nt float2): one damping for all transitions
@@ -187,6 +188,7 @@ cudaError_t launch_adj_fused_reg(UppeHandle* h, int mode, const float2* g, float
                                  StepArgs z_e, StepArgs z_s);
 cudaError_t launch_spec_point(UppeHandle* h, int mode, const float2* C, float2* q_out, float2* qf, const float2* qi,
                               float Cs, float Ce, StepArgs z, const StepArgs* z_next);
+float uppe_em_min(const UppeConfig& c);
 struct TcNext;
 TcNext hankel_tc_next(const UppeHandle* h, StepArgs z_next);
 cudaError_t launch_adj_fused_big(UppeHandle* h, int mode, const float2* g, float2* out, float a_f, float a_mu,
