@@ -79,8 +79,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase, int* er
 
 // Output-tile shapes of the GEMM, one block of 512 threads per multiprocessor: TN = 128 columns per tile and three
 // 64 KB stages; TN = 64 and four 48 KB stages where twice the blocks of the wide tile still fit the chip at once,
-// which shortens a block's copies, products and epilogue: transform with its update, us, wide | narrow: 2049 x 256
-// (66 | 132 blocks) 8.0 | 7.1, 1025 x 256 8.3 | 6.6; 2049 x 512 (132 blocks wide) is slower narrow, every A tile
+// which shortens a block's copies, products and epilogue: one transform by launch list, us, wide | narrow: 2049 x 256
+// (66 | 132 blocks) 8.0 | 7.2, 1025 x 256 (34 | 68) 8.3 | 7.0; 2049 x 512 (132 blocks wide) is slower narrow, every A tile
 // being fetched by twice as many blocks (15.7 | 18.7).  The same bits in both.  A stage is
 // [A_hi | A_lo | B_hi | B_lo]; a B tile of TN rows is the upper or lower half (contiguous 8 KB) of the
 // 128-row split matrix tiles.
@@ -300,7 +300,7 @@ __global__ void __launch_bounds__(TcShape<TN>::THREADS, 1) k_hankel_tc(TcArgs g)
 
 // The pointwise factor on a stored product (in may be out).  As the GEMM's epilogue it ran on the few multiprocessors
 // that have a tile, each point's operands waiting for the stores of the point before: 1025 x 256 (34 blocks), transform
-// with conj(D0) 17.2 us against 8.3 without; apart, a gradient of four steps takes 2.05 ms instead of 2.09.
+// with conj(D0) 17.2 us against 8.3 without; apart 7.0 + 3.9, a gradient of four steps 2.09 -> 2.05 ms.
 template <int CMODE>
 __global__ void __launch_bounds__(256) k_hankel_tc_point(const float2* in, float2* out, OpView op, size_t n, int S,
                                                         StepArgs z) {
