@@ -160,10 +160,11 @@ __global__ void __launch_bounds__(256, TReg<LOGM>::MINB)
         }
         __syncwarp();
         // the soft window on the samples where it is not 1 (wlo at each end), lanes on neighbouring pairs: in the
-        // scan, the end lanes' divisions held the warp up at every step
+        // scan, the end lanes' divisions held the warp up at every step.  A lane takes pair m < M / 2 and its mirror
+        // image, so that each pair has one lane also where the two ends meet (wlo > M)
         const int wlo = tp.wcut + tp.wwid;
 #pragma unroll 1
-        for (int m = t; m < M && 2 * m < wlo; m += TC) {
+        for (int m = t; m < M / 2 && 2 * m < wlo; m += TC) {
 #pragma unroll 1
             for (int end = 0; end < 2; ++end) {
                 const int me = end ? M - 1 - m : m;
