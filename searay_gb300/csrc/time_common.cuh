@@ -38,10 +38,13 @@ struct TimeParams {
 // 1 / x correctly rounded, for normal |x| below 2^126: one Newton step on the hardware's approximation with the
 // residual taken by FMA (P. W. Markstein, IBM J. Res. Dev. 34 (1990) 111).  Equal to __frcp_rn for every
 // significand there, without its branch for the other cases, which keeps the evaluations around it apart.
+// Beyond that range the step gives NaN or nothing and the approximation itself is the result: 0 from 2^126 to
+// infinity, infinity for zero and subnormals (one comparison and a select).
 __device__ __forceinline__ float rcp_normal(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return fmaf(y, fmaf(-x, y, 1.f), y);
+    const float r = fmaf(y, fmaf(-x, y, 1.f), y);
+    return r == r ? r : y;
 }
 
 // Ionization rate in simulation units from the field in simulation units, by the closed form (EXPLICIT) or the
