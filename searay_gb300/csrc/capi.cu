@@ -738,26 +738,6 @@ extern "C" int uppe_set_chi3(UppeHandle* h, double chi3_over_nref) {
     return UPPE_OK;
 }
 
-// In-place FFT of x (length a power of two), sign -1, FP64.
-static void host_fft(std::vector<std::complex<double>>& x) {
-    const size_t n = x.size();
-    for (size_t i = 1, j = 0; i < n; ++i) {
-        size_t bit = n >> 1;
-        for (; j & bit; bit >>= 1) j ^= bit;
-        j ^= bit;
-        if (i < j) std::swap(x[i], x[j]);
-    }
-    std::vector<std::complex<double>> w(n / 2);
-    for (size_t k = 0; k < n / 2; ++k) w[k] = std::polar(1.0, -2.0 * M_PI * (double)k / (double)n);
-    for (size_t len = 2; len <= n; len <<= 1)
-        for (size_t i = 0; i < n; i += len)
-            for (size_t k = 0; k < len / 2; ++k) {
-                const std::complex<double> u = x[i + k], v = x[i + k + len / 2] * w[k * (n / len)];
-                x[i + k] = u + v;
-                x[i + k + len / 2] = u - v;
-            }
-}
-
 extern "C" int uppe_set_rotator(UppeHandle* h, int nstates, const double* Tj, const double* Wj, double dalpha,
                                 double hbar) {
     if (!h || nstates < 0 || (nstates > 0 && (!Tj || !Wj))) {
@@ -778,12 +758,10 @@ extern "C" int uppe_set_rotator(UppeHandle* h, int nstates, const double* Tj, co
         return UPPE_E_ARG;
     }
     if (h->cfg.envelope) {
-        const int keep = h->rot_pairs, keep_conv = h->rot_conv;
+        const int keep = h->rot_pairs;
         h->rot_pairs = ((int)js.size() + 1) / 2;
-        h->rot_conv = 0;  // (the larger of the two forms)
         const size_t need = uppe_env_smem_bytes(h);
         h->rot_pairs = keep;
-        h->rot_conv = keep_conv;
         if (need > 227 * 1024) {
             uppe_set_error(h, "uppe_set_rotator: the envelope time pass would need %zu bytes of shared memory", need);
             return UPPE_E_ARG;
@@ -795,22 +773,13 @@ extern "C" int uppe_set_rotator(UppeHandle* h, int nstates, const double* Tj, co
         h->rot = nullptr;
     }
     h->rot_pairs = 0;
-    h->rot_conv = 0;
     h->E_valid = 0;
     if (js.empty()) return UPPE_OK;
     // transitions in pairs (A, B); an odd count gets a null partner (h2 = 1, cq = 0: adds exactly 0)
     const int npair = ((int)js.size() + 1) / 2, nseg = h->Nt / 16;
     const double dt = h->cfg.dt, Nt = (double)h->Nt;
     // per pair 20 float4: the constants (4) and the powers h2^i, i < 16; then the phasors
-    // and, with one damping rate g >= 0 for all transitions, the tables of the convolution (time_common.cuh), where
-    // the window is shorter than 1/(2 g): a weight that falls further over it would lift the rounding of the
-    // samples at one end over the response at the other
-    const double g2 = 2.0 * Wj[2 * js[0] + 1] * dt;
-    bool conv = g2 >= 0.0 && g2 * Nt <= 1.0;
-    for (int j : js) conv = conv && Wj[2 * j + 1] == Wj[2 * js[0] + 1];
-    const size_t conv_at = (size_t)npair * 80 + (size_t)npair * nseg * 4;
-    std::vector<float> tab(conv_at + (conv ? (size_t)h->Nt * 6 : 0), 0.f);
-    std::vector<double> kern(conv ? h->Nt : 0, 0.0);
+    std::vector<float> tab((size_t)npair * 80 + (size_t)npair * nseg * 4, 0.f);
     for (size_t s = 0; s < 2 * (size_t)npair; ++s) {
         const int pr = (int)(s / 2), lane = (int)(s % 2);
         float* t = &tab[(size_t)80 * pr];
@@ -844,37 +813,11 @@ extern "C" int uppe_set_rotator(UppeHandle* h, int nstates, const double* Tj, co
             t[16 + 4 * i + lane] = (float)hp.real();
             t[16 + 4 * i + 2 + lane] = (float)hp.imag();
         }
-        const std::complex<double> turn = std::polar(std::exp(-0.5 * g2), -wdt.real());
-        std::complex<double> term = cq * std::exp(-0.5 * g2);
-        for (size_t d = 1; d < kern.size(); ++d) {  // Im(cq e^{-i Re(W) dt d}) e^{-g dt (d + 1)}
-            term *= turn;
-            kern[d] += term.imag();
-        }
         // phasor p = e^{i wdt (n + 1/2)} at the first sample n = Nt - 16 (seg + 1) of each segment
         for (int seg = 0; seg < nseg; ++seg) {
             const std::complex<double> p = std::exp(I * wdt * (Nt - 16.0 * (seg + 1) + 0.5));
             p0[4 * seg + lane] = (float)p.real();
             p0[4 * seg + 2 + lane] = (float)p.imag();
-        }
-    }
-    if (conv) {
-        std::vector<std::complex<double>> K(h->Nt);
-        double sum = 0.0;
-        for (int n = 0; n < h->Nt; ++n) {
-            const std::complex<double> ph = std::polar(1.0, 0.5 * M_PI * (double)n / Nt);
-            const double decay = std::exp(-g2 * (double)n);
-            sum += kern[n];
-            K[n] = sum * ph / Nt;
-            float* w = &tab[conv_at + (size_t)2 * n];
-            w[0] = (float)(decay * ph.real());
-            w[1] = (float)(decay * ph.imag());
-            w[2 * h->Nt] = (float)ph.real();
-            w[2 * h->Nt + 1] = (float)ph.imag();
-        }
-        host_fft(K);
-        for (int n = 0; n < h->Nt; ++n) {
-            tab[conv_at + (size_t)4 * h->Nt + 2 * n] = (float)K[n].real();
-            tab[conv_at + (size_t)4 * h->Nt + 2 * n + 1] = (float)K[n].imag();
         }
     }
     void* d = nullptr;
@@ -886,7 +829,6 @@ extern "C" int uppe_set_rotator(UppeHandle* h, int nstates, const double* Tj, co
     h->rot = (float*)d;
     CUDA_TRY(h, cudaMemcpy(h->rot, tab.data(), tab.size() * sizeof(float), cudaMemcpyHostToDevice));
     h->rot_pairs = npair;
-    h->rot_conv = conv ? 1 : 0;
     return UPPE_OK;
 }
 

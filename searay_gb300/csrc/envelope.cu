@@ -25,15 +25,14 @@
 
 namespace {
 
+constexpr int ENV_SPT = 16;  // time samples per thread
+
 __device__ __forceinline__ float cnorm(float2 a) { return fmaf(a.x, a.x, a.y * a.y); }
 
 // Shared layout: ZE [N0][C] (E, then P or chi), ZA [N0][C] (A, then Jpl or ne), the half twiddle
-// table [N0/2], segment totals [2T], then with RAMAN = 1 the Raman chi [N0][C] (float) and the
-// transition tables (20 float4 per pair).  RAMAN = 2: the Raman convolution (time_common.cuh), in ZA while this
-// thread's samples of A wait in registers.
-// SPT: time samples per thread.  With 8, the inverse transforms of E and A (and the forward ones) run side by side,
-// each on half of the threads.
-template <int RAMAN, int SPT>
+// table [N0/2], segment totals [2T], then with RAMAN the Raman chi [N0][C] (float) and the
+// transition tables (20 float4 per pair).
+template <bool RAMAN>
 __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __restrict__ A, float2* __restrict__ out0,
                                                   float2* __restrict__ out1, const float* __restrict__ ng,
                                                   const float* __restrict__ wv, const float2* __restrict__ tw,
@@ -64,7 +63,7 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
     } else {
         for (int k = tid; k < N0; k += T) cp_async8(&ZA[k], &A[(size_t)k * S + col0]);
     }
-    if constexpr (RAMAN == 1)
+    if constexpr (RAMAN)
         for (int i = tid; i < 20 * tp.rot_pairs; i += T) cp_async16_time(&Rs[i], &tp.rot_tab[i]);
     asm volatile("cp.async.commit_group;\n" ::);
     for (int j = tid; j < (N0 >> 1); j += T) twl[j] = __ldg(&tw[j << (twLog - logN0)]);
@@ -72,23 +71,18 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
     __syncthreads();
     for (int it = tid; it < R; it += T) ZE[it] = cmul_i(cscale(ZA[it], __ldg(&wv[it >> logC])));
     __syncthreads();
-    if constexpr (SPT == 8) {
-        const int h = T >> 1;
-        fft_axis_tw<16, RAMAN == 2>(tid < h ? ZE : ZA, logN0, logC, 1, C, tws, true, tid & (h - 1), h);
-    } else {
-        fft_axis_tw<16, RAMAN == 2>(ZE, logN0, logC, 1, C, tws, true, tid, T);
-        fft_axis_tw<16, RAMAN == 2>(ZA, logN0, logC, 1, C, tws, true, tid, T);
-    }
+    fft_axis_tw<16>(ZE, logN0, logC, 1, C, tws, true, tid, T);
+    fft_axis_tw<16>(ZA, logN0, logC, 1, C, tws, true, tid, T);
 
     // ---- 2. sources over this thread's segment t0 .. t0 + 15 of column c ----
     const int c = tid & (C - 1);
     const int seg = tid >> logC;
-    const int t0 = seg * SPT;
+    const int t0 = seg * ENV_SPT;
     const float inv = tp.inv_nt;
     const float ngc = ng[col0 + c];
     const float kerr = 0.75f * ngc * tp.redchi3;
-    if constexpr (RAMAN == 1) {  // F = |z|^2 (the scale (dalpha/hbar)/4/N0^2 is folded into cq)
-        raman_pass<SPT, false>(
+    if constexpr (RAMAN) {  // F = |z|^2 (the scale (dalpha/hbar)/4/N0^2 is folded into cq)
+        raman_pass<ENV_SPT, false>(
             tp, Rs, tot, C, logC, T, tid, seg, ngc,
             [&](int k) { return make_float2(cnorm(ZE[(t0 + 2 * k) * C + c]), cnorm(ZE[(t0 + 2 * k + 1) * C + c])); },
             [&](int k, float chi0, float chi1) {
@@ -96,39 +90,17 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
                 Zr[(t0 + 2 * k + 1) * C + c] = chi1;
             });
     }
-    float2 av[RAMAN == 2 ? SPT : 1];
-    float chr[RAMAN == 2 ? SPT : 1];
-    if constexpr (RAMAN == 2) {
-#pragma unroll
-        for (int i = 0; i < SPT; ++i) av[i] = ZA[(t0 + i) * C + c];
-        __syncthreads();
-        for (int it = tid; it < R; it += T) {
-            const int t = it >> logC, n = N0 - 1 - t;
-            ZA[n * C + c] = cscale(__ldg(&tp.rot_cw[n]), cnorm(ZE[it]));
-        }
-        __syncthreads();
-        fft_axis_tw<SPT, true>(ZA, logN0, logC, 1, C, tws, false, tid, T);
-        for (int it = tid; it < R; it += T) ZA[it] = cmul(ZA[it], __ldg(&tp.rot_cw[2 * N0 + (it >> logC)]));
-        __syncthreads();
-        fft_axis_tw<SPT, true>(ZA, logN0, logC, 1, C, tws, true, tid, T);
-#pragma unroll
-        for (int i = 0; i < SPT; ++i) {
-            const int n = N0 - 1 - t0 - i;
-            const float2 y = ZA[n * C + c], w = __ldg(&tp.rot_cw[N0 + n]);
-            chr[i] = ngc * fmaf(y.x, w.x, y.y * w.y);
-        }
-    }
-    float r[SPT];
+    float r[ENV_SPT];
     float r_next = 0.f;
     ffloat Sacc = {0.f, 0.f};
     if (ionize) {
-        if (t0 + SPT <= N0 - 2) r_next = ion_rate(tp, sqrtf(cnorm(ZE[(t0 + SPT) * C + c])) * inv);
+        if (t0 + ENV_SPT <= N0 - 2) r_next = ion_rate(tp, sqrtf(cnorm(ZE[(t0 + ENV_SPT) * C + c])) * inv);
         ffloat part = {0.f, 0.f};
 #pragma unroll
-        for (int i = SPT - 1; i >= 0; --i) {
+        for (int i = ENV_SPT - 1; i >= 0; --i) {
             const int t = t0 + i;
             r[i] = (t == N0 - 1) ? 0.f : ion_rate(tp, sqrtf(cnorm(ZE[t * C + c])) * inv);
-            const float rn = (i == SPT - 1) ? r_next : r[i + 1];
+            const float rn = (i == ENV_SPT - 1) ? r_next : r[i + 1];
             if (t <= N0 - 2) acc_add(part, tp.hdt * (r[i] + rn), tp.plain);
         }
         const int plain = tp.plain;
@@ -139,23 +111,17 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
     }
     __syncthreads();  // every read of the next segment's first sample (r_next) precedes the writes below
 #pragma unroll
-    for (int i = SPT - 1; i >= 0; --i) {
+    for (int i = ENV_SPT - 1; i >= 0; --i) {
         const int t = t0 + i;
-        const float2 e = cscale(ZE[t * C + c], inv);
-        float2 a;
-        if constexpr (RAMAN == 2)
-            a = cscale(av[i], inv);
-        else
-            a = cscale(ZA[t * C + c], inv);
+        const float2 e = cscale(ZE[t * C + c], inv), a = cscale(ZA[t * C + c], inv);
         float ne = 0.f;
         if (ionize) {
-            const float rn = (i == SPT - 1) ? r_next : r[i + 1];
+            const float rn = (i == ENV_SPT - 1) ? r_next : r[i + 1];
             if (t <= N0 - 2) acc_add(Sacc, tp.hdt * (r[i] + rn), tp.plain);
             ne = ngc * one_minus_exp_neg(ff_value(Sacc));
         }
         float chi = kerr * cnorm(e);
-        if constexpr (RAMAN == 1) chi = Zr[t * C + c] + chi;  // Raman first, then Kerr (paraxial_kernel.py:155-158)
-        if constexpr (RAMAN == 2) chi = chr[i] + chi;
+        if constexpr (RAMAN) chi = Zr[t * C + c] + chi;  // Raman first, then Kerr (paraxial_kernel.py:155-158)
         if (mode == TIME_J) {
             ZE[t * C + c] = cscale(e, chi);
             ZA[t * C + c] = cscale(a, ne * fmaf(0.25f, cnorm(a), -1.f));
@@ -168,16 +134,8 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
 
     // ---- 3. forward FFTs and J = -i w P + Jpl (or the spectra of chi and ne) ----
     const bool two = ionize || mode == TIME_CHI_NE;
-    if constexpr (SPT == 8) {
-        const int h = T >> 1;
-        if (two)
-            fft_axis_tw<16, RAMAN == 2>(tid < h ? ZE : ZA, logN0, logC, 1, C, tws, false, tid & (h - 1), h);
-        else
-            fft_axis_tw<8, RAMAN == 2>(ZE, logN0, logC, 1, C, tws, false, tid, T);
-    } else {
-        fft_axis_tw<16, RAMAN == 2>(ZE, logN0, logC, 1, C, tws, false, tid, T);
-        if (two) fft_axis_tw<16, RAMAN == 2>(ZA, logN0, logC, 1, C, tws, false, tid, T);
-    }
+    fft_axis_tw<16>(ZE, logN0, logC, 1, C, tws, false, tid, T);
+    if (two) fft_axis_tw<16>(ZA, logN0, logC, 1, C, tws, false, tid, T);
     for (int it = tid; it < R; it += T) {
         const int k = it >> logC;
         const size_t o = (size_t)k * S + col0 + (it & (C - 1));
@@ -200,37 +158,25 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
 }  // namespace
 
 cudaError_t uppe_configure_env_kernel(size_t smem_bytes) {
-    cudaError_t e = cudaFuncSetAttribute(k_time_env<0, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+    cudaError_t e = cudaFuncSetAttribute(k_time_env<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_time_env<1, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_time_env<2, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_time_env<2, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+        e = cudaFuncSetAttribute(k_time_env<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     return e;
 }
 
 size_t uppe_env_smem_bytes(const UppeHandle* h) {
-    const size_t R = (size_t)h->Nt * h->time_cols, T = R / (h->rot_conv ? 8 : 16);
+    const size_t R = (size_t)h->Nt * h->time_cols, T = R / 16;
     size_t b = (2 * R + h->Nt / 2) * sizeof(float2) + 2 * T * sizeof(ffloat);
-    if (h->rot_pairs > 0 && !h->rot_conv) b += R * sizeof(float) + (size_t)20 * h->rot_pairs * sizeof(float4);
+    if (h->rot_pairs > 0) b += R * sizeof(float) + (size_t)20 * h->rot_pairs * sizeof(float4);
     return b;
 }
 
 cudaError_t launch_time_env(UppeHandle* h, int mode, const float2* A, float2* out0, float2* out1) {
     const TimeParams tp = uppe_time_params(h);
-    const int R = h->Nt * h->time_cols;
+    const int T = h->Nt * h->time_cols / 16;
     const size_t smem = uppe_env_smem_bytes(h);
-    // the convolution on 8 samples per thread where the block stays within its 512 threads
-    const int form = h->rot_pairs > 0 ? (h->rot_conv ? 2 : 1) : 0;
     h->launches++;
-#define UPPE_ENV_LAUNCH(F_, SPT_)                                                                                      \
-    launch_pdl(k_time_env<F_, SPT_>, dim3(h->S / h->time_cols), dim3(R / SPT_), smem, h->stream, mode, A, out0, out1, \
-               h->ng, h->w, h->tw, h->twLog, tp)
-    if (form == 0) UPPE_ENV_LAUNCH(0, 16);
-    else if (form == 1) UPPE_ENV_LAUNCH(1, 16);
-    else if (R / 8 <= 512 && R >= 32) UPPE_ENV_LAUNCH(2, 8);
-    else UPPE_ENV_LAUNCH(2, 16);
-#undef UPPE_ENV_LAUNCH
+    launch_pdl(h->rot_pairs > 0 ? k_time_env<true> : k_time_env<false>, dim3(h->S / h->time_cols), dim3(T), smem, h->stream,
+               mode, A, out0, out1, h->ng, h->w, h->tw, h->twLog, tp);
     return cudaGetLastError();
 }

@@ -94,13 +94,10 @@ struct RowSwizzle {
     UPPE_DEV int operator()(int e) const { return e ^ (((e & mask) >> sh) & 7); }
 };
 
-// EXACT in the stages below: every twiddle of a radix-8 butterfly from the table (seven loads) instead of three and
-// their products, whose rounding adds to a transform's error as much as its sums do.
-//
 // One radix-R stage over all nb transforms; thread `tid` of `nthr` handles ITEMS butterflies.
 // batch_fast: consecutive threads take consecutive transforms (use when es != 1 so that the
 // accesses of a warp are contiguous in shared memory).
-template <int R, int ITEMS, bool EXACT, class TW, class SW = NoSwizzle>
+template <int R, int ITEMS, class TW, class SW = NoSwizzle>
 UPPE_DEV void stockham_stage(float2* buf, int logN, int logp, int lognb, int bs, int es, const TW& tw, bool inv,
                              bool batch_fast, int tid, int nthr, const SW& sw = SW{}) {
     constexpr int LOGR = (R == 2) ? 1 : (R == 4) ? 2 : 3;
@@ -126,7 +123,7 @@ UPPE_DEV void stockham_stage(float2* buf, int logN, int logp, int lognb, int bs,
         for (int r = 0; r < R; ++r) u[it][r] = base[sw(i + r * nq) * es];
         if (logp > 0) {
             const int sh = tw.log - logp - LOGR;  // NT / (p R)
-            if constexpr (R == 8 && !EXACT) {
+            if constexpr (R == 8) {
                 // W^k, W^2k, W^4k from the table; the other powers as products of at most two of them
                 float2 w1 = tw.get(k << sh), w2 = tw.get((2 * k) << sh), w4 = tw.get((4 * k) << sh);
                 if (inv) {
@@ -166,7 +163,7 @@ UPPE_DEV void stockham_stage(float2* buf, int logN, int logp, int lognb, int bs,
 
 // Full transform along one axis.  ET = elements per thread = nb*N/nthr (compile time); radix 8
 // stages first, then one radix-4 or radix-2 stage for the remainder.
-template <int ET, bool EXACT = false, class TW, class SW = NoSwizzle>
+template <int ET, class TW, class SW = NoSwizzle>
 UPPE_DEV void fft_axis_tw(float2* buf, int logN, int lognb, int bs, int es, const TW& tw, bool inv, int tid,
                           int nthr, int batch_fast_mode = -1, const SW& sw = SW{}) {
     // batch_fast_mode: -1 = automatic (batch-fast when es != 1), 0 = element-fast, 1 = batch-fast
@@ -176,20 +173,20 @@ UPPE_DEV void fft_axis_tw(float2* buf, int logN, int lognb, int bs, int es, cons
         const int rem = logN - logp;
         if constexpr (ET >= 8) {
             if (rem >= 3) {
-                stockham_stage<8, ET / 8, EXACT>(buf, logN, logp, lognb, bs, es, tw, inv, batch_fast, tid, nthr, sw);
+                stockham_stage<8, ET / 8>(buf, logN, logp, lognb, bs, es, tw, inv, batch_fast, tid, nthr, sw);
                 logp += 3;
                 continue;
             }
         }
         if constexpr (ET >= 4) {
             if (rem >= 2) {
-                stockham_stage<4, ET / 4, EXACT>(buf, logN, logp, lognb, bs, es, tw, inv, batch_fast, tid, nthr, sw);
+                stockham_stage<4, ET / 4>(buf, logN, logp, lognb, bs, es, tw, inv, batch_fast, tid, nthr, sw);
                 logp += 2;
                 continue;
             }
         }
         if constexpr (ET >= 2) {
-            stockham_stage<2, ET / 2, EXACT>(buf, logN, logp, lognb, bs, es, tw, inv, batch_fast, tid, nthr, sw);
+            stockham_stage<2, ET / 2>(buf, logN, logp, lognb, bs, es, tw, inv, batch_fast, tid, nthr, sw);
             logp += 1;
         } else {
             break;  // unreachable for valid launches (ET >= 2 whenever logN >= 1)
@@ -225,7 +222,7 @@ UPPE_DEV constexpr RowSwizzle ct_row_swizzle() {
     return RowSwizzle{LOGNB <= 2 ? (1 << LOGN) - 1 : 0, LOGNB == 0 ? 4 : 3};
 }
 
-template <int R, int ITEMS, int LOGN, int LOGP, int LOGNB, int TWLOG, bool EXACT>
+template <int R, int ITEMS, int LOGN, int LOGP, int LOGNB, int TWLOG>
 UPPE_DEV void stockham_stage_ct(float2* buf, const TwHalfSharedCT<TWLOG>& tw, bool inv, int tid) {
     constexpr int LOGR = (R == 2) ? 1 : (R == 4) ? 2 : 3;
     constexpr int NQ = 1 << (LOGN - LOGR), P = 1 << LOGP, NB = 1 << LOGNB;
@@ -243,7 +240,7 @@ UPPE_DEV void stockham_stage_ct(float2* buf, const TwHalfSharedCT<TWLOG>& tw, bo
 #pragma unroll
         for (int r = 0; r < R; ++r) u[it][r] = buf[b + sw(i + r * NQ) * NB];
         if constexpr (LOGP > 0) {
-            if constexpr (R == 8 && !EXACT) {
+            if constexpr (R == 8) {
                 float2 w1 = tw.get(k << SH), w2 = tw.get((2 * k) << SH), w4 = tw.get((4 * k) << SH);
                 if (inv) {
                     w1.y = -w1.y;
@@ -280,19 +277,19 @@ UPPE_DEV void stockham_stage_ct(float2* buf, const TwHalfSharedCT<TWLOG>& tw, bo
     __syncthreads();
 }
 
-template <int ET, int LOGN, int LOGNB, int TWLOG, bool EXACT = false, int LOGP = 0>
+template <int ET, int LOGN, int LOGNB, int TWLOG, int LOGP = 0>
 UPPE_DEV void fft_axis_ct(float2* buf, const TwHalfSharedCT<TWLOG>& tw, bool inv, int tid) {
     if constexpr (LOGP < LOGN) {
         constexpr int REM = LOGN - LOGP;
         if constexpr (ET >= 8 && REM >= 3) {
-            stockham_stage_ct<8, ET / 8, LOGN, LOGP, LOGNB, TWLOG, EXACT>(buf, tw, inv, tid);
-            fft_axis_ct<ET, LOGN, LOGNB, TWLOG, EXACT, LOGP + 3>(buf, tw, inv, tid);
+            stockham_stage_ct<8, ET / 8, LOGN, LOGP, LOGNB, TWLOG>(buf, tw, inv, tid);
+            fft_axis_ct<ET, LOGN, LOGNB, TWLOG, LOGP + 3>(buf, tw, inv, tid);
         } else if constexpr (ET >= 4 && REM >= 2) {
-            stockham_stage_ct<4, ET / 4, LOGN, LOGP, LOGNB, TWLOG, EXACT>(buf, tw, inv, tid);
-            fft_axis_ct<ET, LOGN, LOGNB, TWLOG, EXACT, LOGP + 2>(buf, tw, inv, tid);
+            stockham_stage_ct<4, ET / 4, LOGN, LOGP, LOGNB, TWLOG>(buf, tw, inv, tid);
+            fft_axis_ct<ET, LOGN, LOGNB, TWLOG, LOGP + 2>(buf, tw, inv, tid);
         } else {
-            stockham_stage_ct<2, ET / 2, LOGN, LOGP, LOGNB, TWLOG, EXACT>(buf, tw, inv, tid);
-            fft_axis_ct<ET, LOGN, LOGNB, TWLOG, EXACT, LOGP + 1>(buf, tw, inv, tid);
+            stockham_stage_ct<2, ET / 2, LOGN, LOGP, LOGNB, TWLOG>(buf, tw, inv, tid);
+            fft_axis_ct<ET, LOGN, LOGNB, TWLOG, LOGP + 1>(buf, tw, inv, tid);
         }
     }
 }

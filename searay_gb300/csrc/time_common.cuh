@@ -24,9 +24,6 @@ struct TimeParams {
     int rot_pairs;
     const float4* rot_tab;
     const float4* rot_p0;
-    // the same response as one convolution, with one damping for all transitions (after raman_pass): [3][Nt] weights
-    // in, weights out and the kernel's spectrum
-    const float2* rot_cw;
     // TIME_J with atc set: J goes straight into the split operand tiles of the forward tensor-core
     // Hankel transform (hankel_tc.cuh, azimuthal mode 0) instead of out0
     uint8_t* atc;
@@ -354,21 +351,6 @@ __device__ __forceinline__ void raman_pass(const TimeParams& tp, const float4* R
     __syncthreads();  // `tot` is reused by the density scan
 }
 
-
-// The Raman susceptibility as a convolution.  With one damping rate g for all transitions (Im W_j = g) the sums that
-// raman_pass runs collapse, |p_n| being the same for all of them, to
-//     chi_n = ng sum_{m < n} F_m e^{-2 g dt m} K(n - m),
-//     K(L) = sum_{d=1..L} e^{-g dt (d + 1)} sum_j Im(cq_j e^{-i Re(W_j) dt d}),
-// a linear convolution of Nt samples.  It is taken as a circular one of length Nt with weights e^{i pi n / 2Nt} on
-// both operands (H. J. Nussbaumer, Fast Fourier Transform and Convolution Algorithms, 1982: right-angle circular
-// convolution): what wraps around comes out multiplied by i, so the real part is the linear convolution.  Tables
-// from FP64 on the host, per position n: weights in e^{-2 g dt n} e^{i pi n / 2Nt}, weights out e^{i pi n / 2Nt}, and
-// the spectrum of the weighted K over Nt.
-// Two complex transforms of Nt points replace npair sweeps (15 for N2, two passes over the samples and a block-wide
-// sum each).  With every twiddle from the table (EXACT, fft_smem.cuh) the error of chi against FP64 is, in the mean over
-// 64 to 4096 frequencies, that of the recurrences or below it (1.79e-7 against 1.82e-7 mixed, 2.5e-7 against 2.9e-7
-// FP32, relative L2); from 512 frequencies on it is below at each.
-// N2, 256 columns: time pass 41.4 -> 28.8 us at 4096 samples; envelope 30.6 -> 14.5 us at 256 samples.
 
 // Transpose of raman_pass: the cotangent of the drive F of this thread's SPT consecutive samples
 // (t ascending, index i = t - t0) from the cotangent ybar of the Raman susceptibility at the same

@@ -39,12 +39,11 @@ __device__ __forceinline__ float2 real_spectrum(float2 Za, float2 Zb_raw, float2
 // RAMAN: adds the rotational Raman susceptibility (raman_pass, 16 samples per thread; the segment
 // totals take 2T entries, followed by a third array Zr [M][C] for the Raman chi pairs and the pair
 // tables Rs, 20 float4 per pair).  RAMAN = 1: one block per multiprocessor, F kept in registers;
-// RAMAN = 2: two blocks per multiprocessor.  RAMAN = 3, 4: the same with the Raman convolution (time_common.cuh) in an
-// array of Nt C over Zj and Zr, Zr following Zj; 3: one block per multiprocessor, 4: two.
+// RAMAN = 2: two blocks per multiprocessor.
 template <int ET, int LOGM = 0, int LOGC = -1, int RAMAN = 0>
 // (three blocks per multiprocessor where shared memory allows it: M <= 512)
 __global__ void __launch_bounds__(ET == 16 || (LOGM > 0 && LOGM <= 7) ? 256 : 512,
-                                  RAMAN ? 2 - (RAMAN & 1) : (ET == 16 || (LOGM > 0 && LOGM <= 9) ? 3 : 2)) k_time(int mode, const float2* __restrict__ E, float2* __restrict__ out0,
+                                  RAMAN ? RAMAN : (ET == 16 || (LOGM > 0 && LOGM <= 9) ? 3 : 2)) k_time(int mode, const float2* __restrict__ E, float2* __restrict__ out0,
                                                   float2* __restrict__ out1, const float* __restrict__ ng,
                                                   const float* __restrict__ wv, const float* __restrict__ filt,
                                                   const float2* __restrict__ tw, int twLog, TimeParams tp) {
@@ -54,11 +53,10 @@ __global__ void __launch_bounds__(ET == 16 || (LOGM > 0 && LOGM <= 7) ? 256 : 51
     // column-batched FFT accesses of a warp on distinct banks.
     extern __shared__ float2 Zp[];
     constexpr bool CT = LOGM > 0;
-    constexpr bool RCONV = RAMAN >= 3;
     const int C = CT ? (1 << LOGC) : tp.C, logC = CT ? LOGC : tp.logC;
     const int Nt = CT ? (2 << LOGM) : tp.Nt, M = CT ? (1 << LOGM) : tp.M, S = tp.S;
     float2* Zj = Zp + (size_t)(M + 1) * C;
-    float2* twl = Zj + (size_t)(M + 1) * C + (RCONV ? (size_t)M * C : 0);
+    float2* twl = Zj + (size_t)(M + 1) * C;
     ffloat* tot = reinterpret_cast<ffloat*>(twl + (Nt >> 1));
     const int tid = threadIdx.x, T = CT ? ((2 << LOGM) << LOGC) / (2 * ET) : (int)blockDim.x;
     const size_t col0 = (size_t)blockIdx.x * C;
@@ -84,9 +82,9 @@ __global__ void __launch_bounds__(ET == 16 || (LOGM > 0 && LOGM <= 7) ? 256 : 51
             cp_async8(&Zj[sw(k) * C + c], &E[(size_t)k * S + col0 + c]);
         }
     }
-    float2* Zr = RCONV ? Zj + (size_t)(M + 1) * C : reinterpret_cast<float2*>(tot + 2 * T);
+    float2* Zr = reinterpret_cast<float2*>(tot + 2 * T);
     float4* Rs = reinterpret_cast<float4*>(Zr + (size_t)M * C);
-    if constexpr (RAMAN == 1 || RAMAN == 2)
+    if constexpr (RAMAN != 0)
         for (int i = tid; i < 20 * tp.rot_pairs; i += T) cp_async16_time(&Rs[i], &tp.rot_tab[i]);
     asm volatile("cp.async.commit_group;\n" ::);
     for (int j = tid; j < (Nt >> 1); j += T) twl[j] = __ldg(&tw[j << (twLog - tp.logNt)]);
@@ -114,9 +112,9 @@ __global__ void __launch_bounds__(ET == 16 || (LOGM > 0 && LOGM <= 7) ? 256 : 51
     }
     __syncthreads();
     if constexpr (CT)
-        fft_axis_ct<ET, LOGM, LOGC, LOGM + 1, RCONV>(Zp, TwHalfSharedCT<LOGM + 1>{twl}, true, tid);
+        fft_axis_ct<ET, LOGM, LOGC, LOGM + 1>(Zp, TwHalfSharedCT<LOGM + 1>{twl}, true, tid);
     else
-        fft_axis_tw<ET, RCONV>(Zp, tp.logM, logC, 1, C, tws, true, tid, T, -1, sw);
+        fft_axis_tw<ET>(Zp, tp.logM, logC, 1, C, tws, true, tid, T, -1, sw);
 
     // ---- 2. sources, in place ----
     const int c = tid & (C - 1);
@@ -127,44 +125,7 @@ __global__ void __launch_bounds__(ET == 16 || (LOGM > 0 && LOGM <= 7) ? 256 : 51
     const float ngc = ng[col0 + c];
     const float kerr = ngc * tp.redchi3;
     const float inv = tp.inv_nt;
-    if constexpr (RCONV) {  // F = z^2 at positions n = Nt - 1 - t, eight pairs per thread
-        float2* Zc = Zj;
-        const RowSwizzle sc{logC <= 2 ? Nt - 1 : 0, logC == 0 ? 4 : 3};
-#pragma unroll(CT ? 4 : 1)
-        for (int i = 0; i < 8; ++i) {
-            const int m = (tid + i * T) >> logC, n = Nt - 2 - 2 * m;
-            const float2 zv = Zp[sw(m) * C + c];
-            const float4 w = __ldg(reinterpret_cast<const float4*>(tp.rot_cw + n));  // of positions n and n + 1
-            Zc[sc(n + 1) * C + c] = cscale(make_float2(w.z, w.w), zv.x * zv.x);
-            Zc[sc(n) * C + c] = cscale(make_float2(w.x, w.y), zv.y * zv.y);
-        }
-        __syncthreads();
-        if constexpr (CT)
-            fft_axis_ct<2 * ET, LOGM + 1, LOGC, LOGM + 1, true>(Zc, TwHalfSharedCT<LOGM + 1>{twl}, false, tid);
-        else
-            fft_axis_tw<2 * ET, true>(Zc, tp.logNt, logC, 1, C, tws, false, tid, T, -1, sc);
-#pragma unroll(CT ? 4 : 1)
-        for (int i = 0; i < 16; ++i) {
-            const int k = (tid + i * T) >> logC;
-            Zc[sc(k) * C + c] = cmul(Zc[sc(k) * C + c], __ldg(&tp.rot_cw[2 * Nt + k]));
-        }
-        __syncthreads();
-        if constexpr (CT)
-            fft_axis_ct<2 * ET, LOGM + 1, LOGC, LOGM + 1, true>(Zc, TwHalfSharedCT<LOGM + 1>{twl}, true, tid);
-        else
-            fft_axis_tw<2 * ET, true>(Zc, tp.logNt, logC, 1, C, tws, true, tid, T, -1, sc);
-        float2 chi[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int m = (tid + i * T) >> logC, n = Nt - 2 - 2 * m;
-            const float4 w = __ldg(reinterpret_cast<const float4*>(tp.rot_cw + Nt + n));
-            const float2 y1 = Zc[sc(n + 1) * C + c], y0 = Zc[sc(n) * C + c];
-            chi[i] = make_float2(ngc * fmaf(y1.x, w.z, y1.y * w.w), ngc * fmaf(y0.x, w.x, y0.y * w.y));
-        }
-        __syncthreads();  // Zr lies over the convolution
-#pragma unroll
-        for (int i = 0; i < 8; ++i) Zr[sw((tid + i * T) >> logC) * C + c] = chi[i];
-    } else if constexpr (RAMAN != 0) {  // F = z^2 of the packed pairs z = Nt (E(2m), E(2m+1))
+    if constexpr (RAMAN != 0) {  // F = z^2 of the packed pairs z = Nt (E(2m), E(2m+1))
         raman_pass<16, RAMAN == 1>(
             tp, Rs, tot, C, logC, T, tid, seg, ngc,
             [&](int k) {
@@ -279,11 +240,11 @@ __global__ void __launch_bounds__(ET == 16 || (LOGM > 0 && LOGM <= 7) ? 256 : 51
     // ---- 3. forward FFTs (P, then Jpl) and the current ----
     const bool two = any_ne || mode == TIME_CHI_NE;
     if constexpr (CT) {
-        fft_axis_ct<ET, LOGM, LOGC, LOGM + 1, RCONV>(Zp, TwHalfSharedCT<LOGM + 1>{twl}, false, tid);
-        if (two) fft_axis_ct<ET, LOGM, LOGC, LOGM + 1, RCONV>(Zj, TwHalfSharedCT<LOGM + 1>{twl}, false, tid);
+        fft_axis_ct<ET, LOGM, LOGC, LOGM + 1>(Zp, TwHalfSharedCT<LOGM + 1>{twl}, false, tid);
+        if (two) fft_axis_ct<ET, LOGM, LOGC, LOGM + 1>(Zj, TwHalfSharedCT<LOGM + 1>{twl}, false, tid);
     } else {
-        fft_axis_tw<ET, RCONV>(Zp, tp.logM, logC, 1, C, tws, false, tid, T, -1, sw);
-        if (two) fft_axis_tw<ET, RCONV>(Zj, tp.logM, logC, 1, C, tws, false, tid, T, -1, sw);
+        fft_axis_tw<ET>(Zp, tp.logM, logC, 1, C, tws, false, tid, T, -1, sw);
+        if (two) fft_axis_tw<ET>(Zj, tp.logM, logC, 1, C, tws, false, tid, T, -1, sw);
     }
     for (int it = tid; it < (M + 1) * C; it += T) {
         const int cc = it & (C - 1);
@@ -328,9 +289,7 @@ cudaError_t uppe_configure_time_kernel(size_t smem_bytes) {
 #undef UPPE_TIME_CONF
 #define UPPE_TIME_RCONF(A_, B_)                                                                                     \
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_time<8, A_, B_, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes); \
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_time<8, A_, B_, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes); \
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_time<8, A_, B_, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes); \
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_time<8, A_, B_, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_time<8, A_, B_, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes);
     UPPE_TIME_CT(UPPE_TIME_RCONF)
     UPPE_TIME_RCONF(0, -1)
 #undef UPPE_TIME_RCONF
@@ -407,7 +366,6 @@ TimeParams uppe_time_params(const UppeHandle* h) {
     tp.rot_pairs = h->rot_pairs;
     tp.rot_tab = reinterpret_cast<const float4*>(h->rot);
     tp.rot_p0 = reinterpret_cast<const float4*>(h->rot + 80 * h->rot_pairs);
-    tp.rot_cw = reinterpret_cast<const float2*>(tp.rot_p0 + (size_t)h->rot_pairs * (h->Nt / 16));
     tp.atc = nullptr;
     tp.atc_nwt = tp.atc_nkt = 0;
     if (h->time_atc && h->Atc) {
@@ -433,28 +391,31 @@ cudaError_t launch_time_pass(UppeHandle* h, int mode, const float2* E, float2* o
         TimeParams tr = tp;
         tr.spt = 16;
         const int Tr = h->Nt * h->time_cols / 16;
-        size_t smem_r = ((size_t)(h->M + 1) * 2 * h->time_cols + h->Nt / 2) * sizeof(float2) +
-                        (size_t)2 * Tr * sizeof(ffloat) + (size_t)h->M * h->time_cols * sizeof(float2);
-        if (!h->rot_conv) smem_r += (size_t)20 * h->rot_pairs * sizeof(float4);
-        // two blocks per multiprocessor where their shared memory fits (64 registers, the recurrence's F formed
-        // in each pass), else one block (128 registers, its F held in them)
+        const size_t smem_r = ((size_t)(h->M + 1) * 2 * h->time_cols + h->Nt / 2) * sizeof(float2) +
+                              (size_t)2 * Tr * sizeof(ffloat) + (size_t)h->M * h->time_cols * sizeof(float2) +
+                              (size_t)20 * h->rot_pairs * sizeof(float4);
+        // two blocks per multiprocessor where their shared memory fits (64 registers, F formed in each
+        // pass), else one block with the segment's F held in registers (128 registers)
         const bool occ2 = 2 * (smem_r + 1024) <= (size_t)h->smem_per_sm;
-        const int form = (h->rot_conv ? 3 : 1) + (occ2 ? 1 : 0);
-#define UPPE_TIME_RLAUNCH(A_, B_, F_)                                                                               \
-        launch_pdl(k_time<8, A_, B_, F_>, dim3(h->S / C), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w, \
-                   h->nlfilt, h->tw, h->twLog, tr)
 #define UPPE_TIME_RCASE(A_, B_)                                                                                     \
-        if (A_ == 0 || (tp.logM == A_ && tp.logC == B_)) {                                                            \
-            if (form == 1) UPPE_TIME_RLAUNCH(A_, B_, 1);                                                              \
-            else if (form == 2) UPPE_TIME_RLAUNCH(A_, B_, 2);                                                         \
-            else if (form == 3) UPPE_TIME_RLAUNCH(A_, B_, 3);                                                         \
-            else UPPE_TIME_RLAUNCH(A_, B_, 4);                                                                        \
-            return cudaGetLastError();                                                                                \
+        if (tp.logM == A_ && tp.logC == B_) {                                                                          \
+            if (occ2)                                                                                                 \
+                launch_pdl(k_time<8, A_, B_, 2>, dim3(h->S / h->time_cols), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w, \
+                                                                                 h->nlfilt, h->tw, h->twLog, tr);    \
+            else                                                                                                      \
+                launch_pdl(k_time<8, A_, B_, 1>, dim3(h->S / h->time_cols), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w, \
+                                                                                 h->nlfilt, h->tw, h->twLog, tr);    \
+            return cudaGetLastError();                                                                             \
         }
         UPPE_TIME_CT(UPPE_TIME_RCASE)
-        UPPE_TIME_RCASE(0, -1)
 #undef UPPE_TIME_RCASE
-#undef UPPE_TIME_RLAUNCH
+        if (occ2)
+            launch_pdl(k_time<8, 0, -1, 2>, dim3(h->S / h->time_cols), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w,
+                                                                              h->nlfilt, h->tw, h->twLog, tr);
+        else
+            launch_pdl(k_time<8, 0, -1, 1>, dim3(h->S / h->time_cols), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w,
+                                                                              h->nlfilt, h->tw, h->twLog, tr);
+        return cudaGetLastError();
     }
     if (h->time_spt == 16)
     {

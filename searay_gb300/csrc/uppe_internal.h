@@ -104,7 +104,6 @@ struct UppeHandle {
     float em_min;          // field below which the ionization rate counts as zero (uppe_em_min)
     int rot_pairs;         // rotational Raman transitions in use (uppe_set_rotator), in pairs; 0 = none
     float* rot;            // their tables: [rot_pairs][80] then the phasors [rot_pairs][Nt/16] (float4)
-    int rot_conv;          // the convolution's tables follow (3 Nt float2): one damping for all transitions
     // adjoint work buffers (allocated by the first adjoint call)
     float2 *adj_q1, *adj_q2, *adj_q3, *adj_lf, *adj_acc, *adj_lk, *adj_mu;
     float2* adj_E[4];      // E of the recomputed stage states q0, q1', q2', q3' (reused by the reverse sweep)
