@@ -505,7 +505,7 @@ static cudaError_t eval_to_J(UppeHandle* h, const float2* qsrc, StepArgs z) {
     // cylindrical mixed form, one azimuthal node: J goes straight into the operand tiles of the
     // forward tensor-core transform that follows (its pre-pass is then skipped)
     const bool to_tc = h->cfg.cylindrical && h->cfg.precision == UPPE_PREC_MIXED && h->N2 == 1 && h->tc_next &&
-                       h->Atc;
+                       h->Atc && !h->cfg.envelope;
     h->time_atc = to_tc ? 1 : 0;
     e = launch_time_pass(h, TIME_J, h->E, h->J, nullptr);
     h->time_atc = 0;

@@ -19,7 +19,6 @@
 
 #include "common.cuh"
 #include "fft_smem.cuh"
-#include "hankel_tc.cuh"
 #include "time_common.cuh"
 #include "uppe_internal.h"
 
@@ -50,7 +49,6 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
     const size_t col0 = (size_t)blockIdx.x * C;
     const bool ionize = tp.rate_form != UPPE_RATE_NONE;
     const TwHalfShared tws{twl, logN0};
-    pdl_begin();
 
     // ---- 1. stage A[k][c] (asynchronous copies), then i w A and the two inverse FFTs ----
     if (C >= 2) {
@@ -142,12 +140,7 @@ __global__ void __launch_bounds__(512) k_time_env(int mode, const float2* __rest
         if (mode == TIME_J) {
             float2 J = cmul_mi(cscale(ZE[it], __ldg(&wv[k])));
             if (ionize) J = cadd(J, ZA[it]);
-            if (tp.atc && C > 1)  // the forward tensor-core transform's operand tiles
-                tc_store_pair(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)col0 + (it & (C - 1)), J);
-            else if (tp.atc)
-                tc_store_split(tp.atc, tp.atc_nwt, tp.atc_nkt, 0, k, (int)col0, J);
-            else
-                out0[o] = J;
+            out0[o] = J;
         } else {
             if (out0) out0[o] = ZE[it];
             if (out1) out1[o] = ionize ? ZA[it] : make_float2(0.f, 0.f);
@@ -176,7 +169,9 @@ cudaError_t launch_time_env(UppeHandle* h, int mode, const float2* A, float2* ou
     const int T = h->Nt * h->time_cols / 16;
     const size_t smem = uppe_env_smem_bytes(h);
     h->launches++;
-    launch_pdl(h->rot_pairs > 0 ? k_time_env<true> : k_time_env<false>, dim3(h->S / h->time_cols), dim3(T), smem, h->stream,
-               mode, A, out0, out1, h->ng, h->w, h->tw, h->twLog, tp);
+    if (h->rot_pairs > 0)
+        k_time_env<true><<<h->S / h->time_cols, T, smem, h->stream>>>(mode, A, out0, out1, h->ng, h->w, h->tw, h->twLog, tp);
+    else
+        k_time_env<false><<<h->S / h->time_cols, T, smem, h->stream>>>(mode, A, out0, out1, h->ng, h->w, h->tw, h->twLog, tp);
     return cudaGetLastError();
 }
