@@ -303,7 +303,7 @@ extern "C" int uppe_create(const UppeConfig* cfg, UppeHandle** out) {
     // launch still requests only what its grid needs.
     if (e == cudaSuccess) e = uppe_configure_slice_kernels(227 * 1024);
     if (e == cudaSuccess) e = uppe_configure_time_kernel(227 * 1024);
-    if (e == cudaSuccess && h->tw_reg) e = uppe_configure_time_reg();
+    if (e == cudaSuccess && h->tw_reg) e = uppe_configure_time_reg(227 * 1024);
     if (e == cudaSuccess && h->tw_reg) e = uppe_configure_time_adj_reg();
     if (e == cudaSuccess) e = uppe_configure_time_adj_kernel(224 * 1024);  // leaves room for its static shared memory
     if (e == cudaSuccess && env) e = uppe_configure_env_kernel(227 * 1024);

@@ -377,6 +377,19 @@ TimeParams uppe_time_params(const UppeHandle* h) {
     return tp;
 }
 
+// A grid that can have a multiprocessor for every block asks for more than half of its shared memory, so that no two share
+// one.  On cylindrical grids the chain runs under programmatic launch: the time pass's blocks come while those of the
+// Hankel product still hold their multiprocessors, and are packed two and three to one on those that are free, where
+// each takes longer.  How many are free goes with the product's tiles, so a faster product could make the step slower.
+// Fixed step, us, with 128-column tiles | 64-column ones | these and a block per multiprocessor: 129 x 256 ionizing 114 | 142 |
+// 105, 513 x 512 with 30 Raman transitions 263 | 308 | 232, 1025 x 512 141 | 155 | 138, 4097 x 128 ionizing 315 | 323 |
+// 211, 2049 x 256 160 | 154 | 128; two such handles on two streams 118 | 111, 341 | 241, 226 | 197, 453 | 340 and 223 | 200 without
+// and with it.  Cartesian chains have no such neighbour before the time pass and measure the same either way.
+size_t time_spread_smem(const UppeHandle* h, int blocks, size_t smem) {
+    const size_t half = (size_t)h->smem_per_sm / 2;
+    return h->cfg.cylindrical && blocks <= h->num_sms && smem < half ? half : smem;
+}
+
 cudaError_t launch_time_pass(UppeHandle* h, int mode, const float2* E, float2* out0, float2* out1) {
     if (h->cfg.envelope) return launch_time_env(h, mode, E, out0, out1);
     // the register-resident pass (timepass_reg.cu) for the current J at M = 256, 512, 1024;
@@ -385,7 +398,8 @@ cudaError_t launch_time_pass(UppeHandle* h, int mode, const float2* E, float2* o
     const TimeParams tp = uppe_time_params(h);
     const int C = h->time_cols;
     const int T = h->Nt * C / h->time_spt;
-    const size_t smem = ((size_t)(h->M + 1) * 2 * C + h->Nt / 2) * sizeof(float2) + (size_t)T * sizeof(ffloat);
+    const size_t smem = time_spread_smem(
+        h, h->S / C, ((size_t)(h->M + 1) * 2 * C + h->Nt / 2) * sizeof(float2) + (size_t)T * sizeof(ffloat));
     h->launches++;
     if (h->rot_pairs > 0) {  // 16 samples per thread; Zr and the pair tables after the segment totals
         TimeParams tr = tp;
@@ -397,23 +411,24 @@ cudaError_t launch_time_pass(UppeHandle* h, int mode, const float2* E, float2* o
         // two blocks per multiprocessor where their shared memory fits (64 registers, F formed in each
         // pass), else one block with the segment's F held in registers (128 registers)
         const bool occ2 = 2 * (smem_r + 1024) <= (size_t)h->smem_per_sm;
+        const size_t smem_l = time_spread_smem(h, h->S / C, smem_r);
 #define UPPE_TIME_RCASE(A_, B_)                                                                                     \
         if (tp.logM == A_ && tp.logC == B_) {                                                                          \
             if (occ2)                                                                                                 \
-                launch_pdl(k_time<8, A_, B_, 2>, dim3(h->S / h->time_cols), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w, \
+                launch_pdl(k_time<8, A_, B_, 2>, dim3(h->S / h->time_cols), dim3(Tr), smem_l, h->stream, mode, E, out0, out1, h->ng, h->w, \
                                                                                  h->nlfilt, h->tw, h->twLog, tr);    \
             else                                                                                                      \
-                launch_pdl(k_time<8, A_, B_, 1>, dim3(h->S / h->time_cols), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w, \
+                launch_pdl(k_time<8, A_, B_, 1>, dim3(h->S / h->time_cols), dim3(Tr), smem_l, h->stream, mode, E, out0, out1, h->ng, h->w, \
                                                                                  h->nlfilt, h->tw, h->twLog, tr);    \
             return cudaGetLastError();                                                                             \
         }
         UPPE_TIME_CT(UPPE_TIME_RCASE)
 #undef UPPE_TIME_RCASE
         if (occ2)
-            launch_pdl(k_time<8, 0, -1, 2>, dim3(h->S / h->time_cols), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w,
+            launch_pdl(k_time<8, 0, -1, 2>, dim3(h->S / h->time_cols), dim3(Tr), smem_l, h->stream, mode, E, out0, out1, h->ng, h->w,
                                                                               h->nlfilt, h->tw, h->twLog, tr);
         else
-            launch_pdl(k_time<8, 0, -1, 1>, dim3(h->S / h->time_cols), dim3(Tr), smem_r, h->stream, mode, E, out0, out1, h->ng, h->w,
+            launch_pdl(k_time<8, 0, -1, 1>, dim3(h->S / h->time_cols), dim3(Tr), smem_l, h->stream, mode, E, out0, out1, h->ng, h->w,
                                                                               h->nlfilt, h->tw, h->twLog, tr);
         return cudaGetLastError();
     }

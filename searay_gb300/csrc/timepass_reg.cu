@@ -282,28 +282,32 @@ int time_reg_tables(int M, float2* host) {
 
 size_t time_reg_scratch_len(const UppeHandle* h) { return (size_t)h->S * 2 * (h->M + 1); }
 
-cudaError_t uppe_configure_time_reg() {
-    cudaError_t e = cudaFuncSetAttribute(k_time_reg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TReg<8>::SMEM);
+cudaError_t uppe_configure_time_reg(int smem_bytes) {
+    cudaError_t e = cudaFuncSetAttribute(k_time_reg<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_time_reg<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TReg<9>::SMEM);
+        e = cudaFuncSetAttribute(k_time_reg<9>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_time_reg<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TReg<10>::SMEM);
+        e = cudaFuncSetAttribute(k_time_reg<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
     return e;
 }
 
 cudaError_t launch_time_reg(UppeHandle* h, const float2* E, float2* J) {
     const TimeParams tp = uppe_time_params(h);
     h->launches++;
+#define UPPE_REG_LAUNCH(L_)                                                                                           \
+    launch_pdl(k_time_reg<L_>, dim3(h->S / TReg<L_>::NC), dim3(TReg<L_>::THREADS),                                    \
+               time_spread_smem(h, h->S / TReg<L_>::NC, TReg<L_>::SMEM), h->stream, E, J, h->ng, h->w, h->tw_reg, h->tscr, tp)
     switch (h->M) {
         case 256:
-            launch_pdl(k_time_reg<8>, dim3(h->S / TReg<8>::NC), dim3(TReg<8>::THREADS), TReg<8>::SMEM, h->stream, E, J, h->ng, h->w, h->tw_reg, h->tscr, tp);
+            UPPE_REG_LAUNCH(8);
             break;
         case 512:
-            launch_pdl(k_time_reg<9>, dim3(h->S / TReg<9>::NC), dim3(TReg<9>::THREADS), TReg<9>::SMEM, h->stream, E, J, h->ng, h->w, h->tw_reg, h->tscr, tp);
+            UPPE_REG_LAUNCH(9);
             break;
         default:
-            launch_pdl(k_time_reg<10>, dim3(h->S / TReg<10>::NC), dim3(TReg<10>::THREADS), TReg<10>::SMEM, h->stream, E, J, h->ng, h->w, h->tw_reg, h->tscr, tp);
+            UPPE_REG_LAUNCH(10);
             break;
     }
+#undef UPPE_REG_LAUNCH
     return cudaGetLastError();
 }

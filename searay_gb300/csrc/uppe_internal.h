@@ -143,12 +143,14 @@ cudaError_t launch_fused_cart(UppeHandle* h, int mode, float Cs, float Ce, StepA
 // Cartesian first stage from k1 (adaptive step) fused with the inverse transform to E.
 cudaError_t launch_apply1_cart(UppeHandle* h, float Cs, float Ce, StepArgs z);
 cudaError_t launch_time_pass(UppeHandle* h, int mode, const float2* E, float2* out0, float2* out1);
+// Dynamic shared memory to ask for a time pass of `blocks` blocks that need `smem` bytes (timepass.cu).
+size_t time_spread_smem(const UppeHandle* h, int blocks, size_t smem);
 // register-resident time pass (timepass_reg.cu): TIME_J for M = 256, 512, 1024 without a rotator
 bool time_reg_supported(const UppeHandle* h);
 size_t time_reg_table_len(int M);
 int time_reg_tables(int M, float2* host);
 size_t time_reg_scratch_len(const UppeHandle* h);
-cudaError_t uppe_configure_time_reg();
+cudaError_t uppe_configure_time_reg(int smem_bytes);
 cudaError_t launch_time_reg(UppeHandle* h, const float2* E, float2* J);
 // register-resident adjoint time pass (timepass_adj_reg.cu): the columns without ionization
 int time_adj_reg_group(int M);
