@@ -414,8 +414,11 @@ extern "C" int uppe_set_grid(UppeHandle* h, const double* w, const double* kr2, 
             if (!h->Atc) {
                 h->Atc_bytes = uppe_hankel_tc_atile_bytes(h->N0, Nr, Nm);
                 CUDA_TRY(h, cudaMalloc((void**)&h->Atc, h->Atc_bytes));
-                // the padding of the tiles (w >= N0, k >= N1) stays zero: the kernels that write the
-                // tiles directly (time pass, spectral update) write only inside the grid
+                // N1 is a power of two, so a transform over the radial nodes has whole tiles of 64, or one whose
+                // columns from N1 on are zero from here: the kernels that write tiles directly (time passes, azimuthal
+                // DFT, spectral update) write only inside the grid, and the transform's own pre-pass writes zeros there.
+                // Beyond the Nk modes the spectral update and the pre-pass write zeros each time.  Rows from N0 on may hold
+                // anything: they only reach outputs that are not stored.
                 CUDA_TRY(h, cudaMemset(h->Atc, 0, h->Atc_bytes));
             }
         }

@@ -315,7 +315,7 @@ static cudaError_t launch_azimuth_tiles(UppeHandle* h, const float2* in) {
     const int logN2 = ilog2_exact(h->N2);
     const size_t n = ((((size_t)h->N0 * h->N1 + 7) >> 3) << 3) * h->N2;
     unsigned blocks = (unsigned)((n + 255) / 256);
-    if (blocks > 152 * 16) blocks = 152 * 16;
+    if (blocks > 16u * h->num_sms) blocks = 16u * h->num_sms;
     h->launches++;
     h->atc_next = 0;
     k_azimuth_tiles<<<blocks, 256, 0, h->stream>>>(in, h->Atc, h->N0, h->N1, h->N2, logN2, (h->N0 + TC_W - 1) / TC_W,
@@ -431,9 +431,7 @@ cudaError_t launch_spec_cyl(UppeHandle* h, int mode, const float2* src_real, flo
     g.A = src_real;
     if (h->N2 > 1) {
         g.A = h->scratch;
-        // (a ragged last tile needs the zeros that the transform's own pre-pass writes, unless it is the only one)
-        const bool tiles = h->cfg.precision == UPPE_PREC_MIXED && h->tc_next && h->Atc &&
-                           (h->N1 % TC_K == 0 || h->N1 < TC_K);
+        const bool tiles = h->cfg.precision == UPPE_PREC_MIXED && h->tc_next && h->Atc;
         cudaError_t err = tiles ? launch_azimuth_tiles(h, src_real) : launch_azimuth(h, src_real, h->scratch, false);
         if (err != cudaSuccess) return err;
         if (tiles) {

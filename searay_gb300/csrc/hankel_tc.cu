@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(256) k_hankel_tc_point(const float2* in, float
 template <int CMODE>
 static cudaError_t run_point(UppeHandle* h, const float2* in, float2* out, StepArgs z) {
     size_t blocks = (h->P + 255) / 256;
-    if (blocks > 152 * 8) blocks = 152 * 8;
+    if (blocks > (size_t)8 * h->num_sms) blocks = (size_t)8 * h->num_sms;
     h->launches++;
     launch_pdl(k_hankel_tc_point<CMODE>, dim3((unsigned)blocks), dim3(256), 0, h->stream, in, out, uppe_op_view(h), h->P,
                h->S, z);
