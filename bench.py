@@ -674,7 +674,7 @@ def main():
     if rank == 0 and not args.no_e2e:
         e2e, h2d, d2h, ok, n_e2e = run_e2e(args, vd, args.precision)
         line["e2e"] = {"value": e2e * ws, "unit": UNIT, "h2d_bytes_per_step": h2d / n_e2e,
-                       "d2h_bytes_per_step": d2h / n_e2e, "steps": n_e2e,
+                       "d2h_bytes_per_step": d2h / n_e2e, "steps": n_e2e, "finite": ok,
                        "call": "searay_gb300.track (host NumPy in/out), one call over the steps"}
     if rank == 0 and not args.no_cpu_baseline and ws == 1:
         base, v_sample, ref = cpu_baseline(vd, outputs=True)
