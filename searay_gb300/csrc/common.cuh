@@ -193,7 +193,7 @@ UPPE_DEV float2 propagator_factor(const OpPoint& o, PhaseArgs pa, float sign) {
 // The two propagator factors of a stage update in the usual case, known when the kernel is chosen: the mixed
 // form in a real medium (float-float phase, Im kz = 0).  The branches of propagator_factor and its
 // full-range sincos and exp then leave the kernel, and where both factors are at the same z (`same`, half
-// of the stage updates) one phasor serves both.  The same bits as the general form gives there.
+// of the stage updates) one phasor serves both.  The same FP32 expressions as the general form, to their rounding.
 struct PropagatorPair {
     float c, s;  // exp(i(kz + kg) z) at the last z asked
     // exp(-i(kz + kg) z) a

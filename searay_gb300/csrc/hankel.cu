@@ -43,11 +43,11 @@ struct GemmArgs {
 // epilogue's code exists once (unrolled over a thread's products it stalled on instruction fetch), its
 // accesses are coalesced, and its operands are loaded four points ahead of the stores.
 //
-// Bound by the FMA pipe: at 2049 x 512 x 512 a product is 1.07e9 FMAs, 28 us at the 39e12/s of 152
-// multiprocessors, about 40 us at the rate an outer product in registers reaches.  Measured there, the propagator
-// factor or the RK stage included: 68 us, against 127 and 120 us with 32 x 64 tiles of 2 x 4 and no copies
-// ahead (512 threads of 2 x 8 against 256 of 4 x 8: 68 against 71 us; scalar FMAs in place of packed
-// ones: the same).
+// At 2049 x 512 x 512 a product is 1.07e9 FMAs, 28 us at the 39e12/s of 152 multiprocessors.  Bound by the delivery of
+// its operands from shared memory (L1 pipe 70 % busy, `mio_throttle` and `short_scoreboard` the top stalls, issue
+// 46 to 52 % on 130 blocks).  Measured there, the propagator factor or the RK stage included: 67 and 70 us, against
+// 127 and 120 us with 32 x 64 tiles of 2 x 4 and no copies ahead (512 threads of 2 x 8 against 256 of 4 x 8: 68 against
+// 71 us; scalar FMAs in place of packed ones: the same).
 template <int BM, int BN, int TM, int TN>
 struct GemmShape {
     static constexpr int TX = BN / TN, TY = BM / TM, T = TX * TY, AE = BM * GBK / T, BE = GBK * BN / 4 / T;

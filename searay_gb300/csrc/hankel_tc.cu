@@ -80,9 +80,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t phase, int* er
 // Output-tile shapes of the GEMM, one block of 512 threads per multiprocessor: TN = 128 columns per tile and three
 // 64 KB stages; TN = 64 and four 48 KB stages where twice the blocks of the wide tile still fit the chip at once,
 // which shortens a block's copies, products and epilogue: one transform by launch list, us, wide | narrow: 2049 x 256
-// (66 | 132 blocks) 8.0 | 7.2, 1025 x 256 (34 | 68) 8.3 | 7.0; 2049 x 512 (132 blocks wide) is slower narrow, every A tile
-// being fetched by twice as many blocks (15.7 | 18.7).  The same bits in both.  A stage is
-// [A_hi | A_lo | B_hi | B_lo]; a B tile of TN rows is the upper or lower half (contiguous 8 KB) of the
+// (66 | 132 blocks) 8.0 | 7.2, 1025 x 256 (34 | 68) 8.3 | 7.0; at 2049 x 512 (132 | 264 blocks, two waves narrow) 10.8 | 17.4,
+// a fixed step 207 | 257.  The same bits in both.  (What the time pass after it makes of the occupied multiprocessors:
+// time_spread_smem, timepass.cu.)  A stage is [A_hi | A_lo | B_hi | B_lo]; a B tile of TN rows is the upper or lower half (contiguous 8 KB) of the
 // 128-row split matrix tiles.
 template <int TN>
 struct TcShape {

@@ -451,8 +451,8 @@ UPPE_DEV void stage_async16(float2* smem_dst, const float2* gsrc) {
 // the pointwise operands stream through the ring during the forward transform and the pointwise
 // loop.
 //
-// Bound by instruction issue (68 % of the issue slots, 262 thread instructions per point at 128 x 128,
-// about 100 of them pointwise).  FAST (PropagatorPair: the mixed form in a real medium) takes the branches,
+// Bound by instruction issue (62 % of the issue slots, `not_selected` the top stall, 294 thread instructions per point
+// at 128 x 128; the general form 68 % and 354).  FAST (PropagatorPair: the mixed form in a real medium) takes the branches,
 // the full-range sincos and exp and half of the phasors of two of the four stages out of the loop, and
 // with that shorter body four registers a trip pay off: 513 x 128 x 128, the pass with its zero-current
 // slices 117.8 -> 107.1 us per evaluation (FAST alone 110.5, with ROT = 4 108.9).  The general form keeps ROT = 2.
